@@ -591,6 +591,45 @@ int Engine::add_bcsr(const b4csr_matrix_if& b, int method)
     return CSP_OK;
 }
 
+// The blocks of a generic BCSR as records (BlockRec in kernels/spmm.cuh): the caller's
+// element planes are copied a slice at a time and turned into records on the device (on
+// the host the same took as long again as the upload); zero records follow the last block.
+int Engine::upload_block_records(Part& p, const bcsr_matrix_if& b)
+{
+    const int bs = p.bw * p.bh;
+    const size_t al = (size_t)b.bcsr_aligned_size, nblk = (size_t)b.bcsr_block_num, es = bf16 ? 2 : 4;
+    const size_t words = dev::record_words(bs, bf16);
+    int rc = alloc(&p.v, (nblk + dev::kSpmmPadBlocks) * words * 4);
+    if (rc) return rc;
+    CSP_CUDA(cudaMemset(static_cast<uint32_t*>(p.v) + nblk * words, 0, (size_t)dev::kSpmmPadBlocks * words * 4));
+    p.records = true;
+    if (!nblk) return CSP_OK;
+    const size_t slice = std::min<size_t>(nblk, (size_t)4 << 20);
+    // slice layout: the columns, then the bs planes
+    char* tmp = nullptr;
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&tmp), slice * (4 + bs * es));
+    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (block records)");
+    std::vector<uint16_t> t(bf16 ? slice : 0);
+    for (size_t j = 0; j < nblk && e == cudaSuccess; j += slice) {
+        const size_t n = std::min(slice, nblk - j);
+        e = cudaMemcpy(tmp, b.bcsr_col_id + j, n * 4, cudaMemcpyHostToDevice);
+        for (int q = 0; q < bs && e == cudaSuccess; q++) {
+            const float* src = b.bcsr_data + q * al + j;
+            if (bf16)
+                for (size_t i = 0; i < n; i++) t[i] = to_bf16(src[i]);
+            e = cudaMemcpy(tmp + slice * 4 + q * slice * es, bf16 ? static_cast<const void*>(t.data()) : src, n * es,
+                           cudaMemcpyHostToDevice);
+        }
+        if (e != cudaSuccess) break;
+        dev::block_records_kernel<<<grid_for((long long)n, 256), 256>>>(reinterpret_cast<const int*>(tmp), tmp + slice * 4,
+                                                                       static_cast<uint32_t*>(p.v) + j * words, (int)n, (int)slice,
+                                                                       bs, bf16, nrhs / 4);
+        e = cudaGetLastError();
+    }
+    cudaFree(tmp);   // waits for the last slice's kernel
+    return e == cudaSuccess ? CSP_OK : cuda_error(e, "block records");
+}
+
 int Engine::add_generic_bcsr(const bcsr_matrix_if& b, int method)
 {
     const unsigned bw = b.bcsr_bwidth, bh = b.bcsr_bheight;
@@ -631,7 +670,10 @@ int Engine::add_generic_bcsr(const bcsr_matrix_if& b, int method)
         fits = fits && !work.empty();
     }
     const int nblk = b.bcsr_block_num;
-    if (!fits) {
+    if (nrhs % 4 == 0 && !(tensor_spmm && nrhs % 32 == 0 && bw * bh <= 16)) {
+        // several right-hand sides in whole float4s: block records (kernels/spmm.cuh)
+        if ((rc = upload_block_records(p, b))) return rc;
+    } else if (!fits) {
         if ((rc = upload_int(&p.i1, b.bcsr_col_id, nblk, (size_t)pad_to(nblk, 4) + 4)) ||
             (rc = upload_val(&p.v, b.bcsr_data, nd, nd)))
             return rc;
@@ -714,25 +756,36 @@ static void launch_spmm(const Part& p, const float* x, float* y, int n, int k, b
         case 16: csr_spmm_kernel<V, 16><<<g, kSpmmThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.m, k); break;
         default: csr_spmm_kernel<V, 32><<<g, kSpmmThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.m, k); break;
         }
-    } else if (p.kind == PART_GBCSR && k % 4 == 0) {
-        // register-blocked: CW lanes x 4 right-hand sides, 4 sub-groups over the blocks
+    } else if (p.kind == PART_GBCSR && p.records) {
+        const unsigned* rec = static_cast<const unsigned*>(p.v);
         if (p.nbr == 0) return;
-        const int CW = k >= 32 ? 8 : (k >= 16 ? 4 : (k >= 8 ? 2 : 1));
-        const unsigned g = grid_for((long long)p.nbr * CW * 4, kSpmmThreads);
+        // float4 columns per pass: all of k up to 32, so A is read once
+        const int CW = k > 16 ? 8 : (k > 8 ? 4 : (k > 4 ? 2 : 1));
+#define CSP_GB4K(BH, BW, C, K)                                                                                                   \
+    do {                                                                                                                         \
+        using Sh = SpmmShape<V, BH, BW, C>;                                                                                      \
+        /* as many block rows per lane group as one wave of resident groups needs, up to max_rows: */                            \
+        /* 20,000 block rows at k = 20 in 1.06 waves of 4 rows take 27.0 us, in one wave of 5 rows 22.9 */                          \
+        const int wave = 148 * Sh::ctas * Sh::warps * Sh::groups;                                                                \
+        const int rows = std::min(Sh::max_rows, (p.nbr + wave - 1) / wave);                                                      \
+        const long long ng = ((long long)p.nbr + rows - 1) / rows;                                                               \
+        bcsr_spmm_stream_kernel<V, BH, BW, C, K><<<grid_for(ng * Sh::GL, Sh::threads), Sh::threads, 0, st>>>(                    \
+            p.i0, rec, x, y, p.nbr, p.m, k, rows);                                                                               \
+    } while (0)
 #define CSP_GB4(BH, BW)                                                                                                          \
     do {                                                                                                                         \
-        switch (CW) {                                                                                                            \
-        case 1: bcsr_spmm4_kernel<V, BH, BW, 1, 4><<<g, kSpmmThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.nbr, p.stride, p.m, n, k); break; \
-        case 2: bcsr_spmm4_kernel<V, BH, BW, 2, 4><<<g, kSpmmThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.nbr, p.stride, p.m, n, k); break; \
-        case 4: bcsr_spmm4_kernel<V, BH, BW, 4, 4><<<g, kSpmmThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.nbr, p.stride, p.m, n, k); break; \
-        default: bcsr_spmm4_kernel<V, BH, BW, 8, 4><<<g, kSpmmThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.nbr, p.stride, p.m, n, k); break; \
-        }                                                                                                                        \
+        if (CW == 1) CSP_GB4K(BH, BW, 1, 4);                                                                                     \
+        else if (CW == 2) CSP_GB4K(BH, BW, 2, 8);                                                                                \
+        else if (CW == 4) CSP_GB4K(BH, BW, 4, 0);                                                                                \
+        else if (k == 32) CSP_GB4K(BH, BW, 8, 32);                                                                               \
+        else CSP_GB4K(BH, BW, 8, 0);                                                                                             \
     } while (0)
         switch (p.bh * 10 + p.bw) {
         case 11: CSP_GB4(1, 1); break; case 22: CSP_GB4(2, 2); break; case 33: CSP_GB4(3, 3); break;
         case 44: CSP_GB4(4, 4); break; case 66: CSP_GB4(6, 6); break;
         }
 #undef CSP_GB4
+#undef CSP_GB4K
     } else if (p.kind == PART_GBCSR) {
         if (p.nbr == 0) return;
         const unsigned g = grid_for((long long)p.nbr * G, kSpmmThreads);

@@ -37,6 +37,7 @@ struct Part {
     int maxw = 0;     // BDIA widest band
     int group = 0;    // CSR sub-warp lanes per row
     int nblocks = 0;  // CSR adaptive row blocks
+    bool records = false;  // generic BCSR, k % 4 == 0: v holds block records (kernels/spmm.cuh)
     int npad = 0, nwarps = 0;  // COO
     // x-panel layout (kernels/xpanel.cuh): i0 = run slot per entry, v = values
     unsigned short* lcol = nullptr;   // column inside the entry's panel
@@ -123,6 +124,7 @@ struct Engine {
     int add_bell(const b4ell_matrix_if& b, int method);
     int add_sbell(const sbell_matrix_if& s, int method);
     int add_bcsr(const b4csr_matrix_if& b, int method);
+    int upload_block_records(Part& p, const bcsr_matrix_if& b);
     int add_generic_bcsr(const bcsr_matrix_if& b, int method);
 };
 

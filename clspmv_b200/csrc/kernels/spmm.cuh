@@ -103,113 +103,247 @@ __global__ void __launch_bounds__(kSpmmThreads) bcsr_spmm_kernel(const int* __re
     }
 }
 
-// Generic BCSR with k a multiple of 4: register-blocked.  A block row is served by
-// L = CW * S lanes: CW lanes each own 4 consecutive right-hand sides (128-bit loads of
-// X and Y rows) and S sub-groups split the block row's blocks, summed by shuffles at
-// the end.  Block values are staged element-major -> shared memory by coalesced loads
-// (one block per lane of the group) and read back as broadcasts.  Columns beyond
-// 4 * CW are handled in further passes.
-template <class V, int BH, int BW, int CW, int S>
-__global__ void __launch_bounds__(kSpmmThreads) bcsr_spmm4_kernel(const int* __restrict__ rp, const int* __restrict__ col,
-                                                                  const V* __restrict__ data, const float* __restrict__ x,
-                                                                  float* __restrict__ y, int nbr, int aligned, int m, int n,
-                                                                  int k)
+// Generic BCSR with k a multiple of 4, on a layout of its own: block j is BlockRec<V, BS>
+// words -- its BS values in row-major order (two per word in BF16), then the index of
+// its first X row in float4s -- so a run of blocks is one contiguous stream.  A warp is
+// cut into groups of GL = 4 CW lanes; a group takes `rows` consecutive block rows one
+// after the other and copies their blocks through a ring of four chunks in shared memory
+// with 16-byte cp.async, two chunks ahead.  Per step a group takes 4 U blocks of its
+// current row: lane (cw, sub) owns right-hand sides 4 cw .. 4 cw + 3 of blocks sub,
+// sub + 4, ..., whose X loads are all in flight together.  At the end of a row the four
+// lanes of a column are summed by two shuffle steps that also split the four right-hand
+// sides over them, so Y is read (when the row begins) and written by whole segments of
+// consecutive lanes.
+//
+// What bounds it: the X rows.  Every block reads BW * k floats of X from L2 (384 bytes at
+// 3x3, k = 32; the band of a FEM matrix is too wide for L1), so the floor is the L2 -> SM
+// path and the L1 tag rate (BW lines a block at a line a clock), not HBM; next to it, issue
+// slots: BH * BW * 4 FMAs per lane and block, and as few other instructions as possible --
+// no predicated loads (lanes past the row's end read X row 0 and skip the products).
+// Measured (500,000 block rows, 10 M 3x3 blocks, one B200): k = 32 FP32 615 -> 343 us, k = 16
+// 530 -> 271, k = 8 BF16 250 -> 187, k = 4 FP32 245 -> 182 (before: blocks staged row by row
+// from the element planes, one barrier pair per 32 blocks, ~880 instructions a block row at
+// k = 32; now ~580).  The X gathers alone take 192 us at k = 32.  Also measured at k = 32:
+// one round of X loads in flight (U = 1) 406 us, 24 warps an SM 403, 48 warps with U = 1 482;
+// X rows copied to shared memory by cp.async.bulk 250 us for the gathers alone; a block's
+// three X rows read as one request over 6 lanes, 227 us at k = 8 (three FMA sets for one).
+template <class V, int BS> struct BlockRec {
+    static constexpr int value_words = sizeof(V) == 4 ? BS : (BS + 1) / 2;
+    static constexpr int align = value_words >= 8 ? 4 : 2;    // words of one shared-memory read
+    static constexpr int words = (value_words + align) / align * align;
+    static constexpr int xrow_word = words - 1;
+};
+// BlockRec<V, bs>::words
+inline size_t record_words(int bs, bool bf16)
 {
-    constexpr int BS = BH * BW;
-    constexpr int L = CW * S;
-    __shared__ float s_val[kSpmmThreads * BS];
-    __shared__ int s_col[kSpmmThreads];
-    const int lane = threadIdx.x % L;
+    const int value_words = bf16 ? (bs + 1) / 2 : bs, align = value_words >= 8 ? 4 : 2;
+    return (size_t)(value_words + align) / align * align;
+}
+
+// Records of n blocks from their columns and element planes (plane q at q * stride
+// elements); set-up only.  x_units: float4s per X row.
+__global__ void __launch_bounds__(256) block_records_kernel(const int* __restrict__ col, const void* __restrict__ planes,
+                                                            unsigned* __restrict__ rec, int n, int stride, int bs, bool bf16,
+                                                            int x_units)
+{
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    if (j >= n) return;
+    const int value_words = bf16 ? (bs + 1) / 2 : bs, align = value_words >= 8 ? 4 : 2;
+    const int words = (value_words + align) / align * align;
+    unsigned* r = rec + (size_t)j * words;
+    for (int i = 0; i < words - 1; i++) {
+        unsigned v = 0u;
+        if (i < value_words) {
+            if (bf16) {
+                const unsigned short* s = static_cast<const unsigned short*>(planes);
+                v = s[(size_t)(2 * i) * stride + j];
+                if (2 * i + 1 < bs) v |= (unsigned)s[(size_t)(2 * i + 1) * stride + j] << 16;
+            } else {
+                v = static_cast<const unsigned*>(planes)[(size_t)i * stride + j];
+            }
+        }
+        r[i] = v;
+    }
+    r[words - 1] = (unsigned)col[j] * (unsigned)x_units;
+}
+
+constexpr int kSpmmPadBlocks = 32;   // zero records behind the last block: a chunk may be copied past its end
+
+// values of a block record in shared memory
+template <class V, int BS>
+__device__ __forceinline__ void read_block(const unsigned* s, float (&a)[BS])
+{
+    using Rec = BlockRec<V, BS>;
+    unsigned wd[(Rec::value_words + 3) / 4 * 4];
+    if (Rec::align == 4) {
+#pragma unroll
+        for (int i = 0; i < (Rec::value_words + 3) / 4; i++) {
+            const uint4 u = *reinterpret_cast<const uint4*>(s + 4 * i);
+            wd[4 * i] = u.x;
+            wd[4 * i + 1] = u.y;
+            wd[4 * i + 2] = u.z;
+            wd[4 * i + 3] = u.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < (Rec::value_words + 1) / 2; i++) {
+            const uint2 u = *reinterpret_cast<const uint2*>(s + 2 * i);
+            wd[2 * i] = u.x;
+            wd[2 * i + 1] = u.y;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < BS; q++) {
+        if (sizeof(V) == 4) a[q] = __uint_as_float(wd[q]);
+        else a[q] = __uint_as_float(q % 2 ? wd[q / 2] & 0xffff0000u : wd[q / 2] << 16);
+    }
+}
+
+// The lane split for CW float4 columns a pass.
+template <class V, int BH, int BW, int CW> struct SpmmShape {
+    static constexpr int BS = BH * BW;
+    static constexpr int GL = 4 * CW, groups = 32 / GL;
+    // rounds of X loads in flight: two, where 64 registers hold them; at one float4 column
+    // (k = 4) one, which halves the ring and keeps more warps resident (197 -> 182 us)
+    static constexpr int U = BW > 4 || CW == 1 ? 1 : 2;
+    static constexpr int chunk = 4 * U > 2 * CW ? 4 * U : 2 * CW;               // blocks; a step spans at most two
+    static constexpr int ring_words = 4 * chunk * BlockRec<V, BS>::words;       // per group
+    static constexpr int warp_bytes = groups * ring_words * 4;
+    static constexpr int warps = warp_bytes * 8 <= 48 * 1024 ? 8 : (warp_bytes * 4 <= 48 * 1024 ? 4 : (warp_bytes * 2 <= 48 * 1024 ? 2 : 1));
+    static constexpr int threads = 32 * warps;
+    // consecutive block rows per group: a warp per row needs eight to hide the start of its ring
+    static constexpr int max_rows = groups == 1 ? 8 : 4;
+    static constexpr int ctas = (BS <= 9 ? 32 : (BS <= 16 ? 24 : 16)) / warps;   // per SM
+};
+
+// K: the number of right-hand sides where it is known (0: `k_arg`).
+template <class V, int BH, int BW, int CW, int K>
+__global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V, BH, BW, CW>::ctas)
+    bcsr_spmm_stream_kernel(const int* __restrict__ rp, const unsigned* __restrict__ rec, const float* __restrict__ x,
+                            float* __restrict__ y, int nbr, int m, int k_arg, int rows)
+{
+    using Sh = SpmmShape<V, BH, BW, CW>;
+    using Rec = BlockRec<V, BH * BW>;
+    constexpr int BS = BH * BW, GL = Sh::GL, U = Sh::U, CH = Sh::chunk, NW = Rec::words;
+    constexpr int RM = 4 * CH - 1;   // ring index mask
+    static_assert((CH & (CH - 1)) == 0 && CH * NW % 4 == 0, "ring of a power of two blocks, whole 16-byte copies");
+    __shared__ __align__(16) unsigned s_ring[32 * Sh::warps / GL][Sh::ring_words];
+    const int k = K ? K : k_arg;
+    const int lane = threadIdx.x % GL;                       // in the group
+    unsigned* ring = s_ring[threadIdx.x / GL];
+    const unsigned ring_addr = (unsigned)__cvta_generic_to_shared(ring);
+    const int gid = (int)(((long long)blockIdx.x * Sh::threads + threadIdx.x) / GL);
+    const int r0 = (int)min((long long)gid * rows, (long long)nbr), r1 = min(r0 + rows, nbr);
     const int cw = lane % CW, sub = lane / CW;
-    const int gbase = threadIdx.x - lane;
-    const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << ((threadIdx.x & 31) - lane));
-    const int br = (int)(((long long)blockIdx.x * kSpmmThreads + threadIdx.x) / L);
-    const bool valid = br < nbr;
-    const int s = valid ? __ldg(rp + br) : 0, e = valid ? __ldg(rp + br + 1) : 0;
+    const int rend = __ldg(rp + min(r0 + 1 + lane, r1));     // rows <= GL: the ends of the group's rows
+    const int sb = __ldg(rp + r0), eb = __ldg(rp + r1);
+    const int base = sb & ~1;                                // chunks start on 16 bytes
+    // the right-hand side of this lane's results: c + comp
+    const int comp = ((lane & CW) ? 2 : 0) + ((lane & (2 * CW)) ? 1 : 0);
+    const size_t kb = (size_t)k * 4;
+
+    // chunk q of the group's blocks into ring slot q % 4
+    auto issue = [&](int q) {
+        const int j = base + q * CH;
+        if (j < eb) {
+            const char* src = reinterpret_cast<const char*>(rec + (size_t)j * NW);
+            const unsigned dst = ring_addr + (q & 3) * (CH * NW * 4);
+#pragma unroll
+            for (int i = 0; i < CH * NW / 4; i += GL)
+                if (i + lane < CH * NW / 4)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * (i + lane)),
+                                 "l"(src + 16 * (i + lane)));
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+
     for (int c0 = 0; c0 < k; c0 += 4 * CW) {
         const int c = c0 + 4 * cw;
-        const bool active = c < k;
+        const bool writer = c < k;
+        const char* __restrict__ xc = reinterpret_cast<const char*>(x + (c < k ? c : 0));
+        float* __restrict__ yp = y + (size_t)r0 * BH * k + c + comp;   // this lane's Y entry of the row's first line
+        issue(0);
+        issue(1);
+        int next = 0;               // chunks 0 .. next - 1 have landed
+        int j = sb, r = r0, re = sb;
         float4 acc[BH];
-#pragma unroll
-        for (int h = 0; h < BH; h++) acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-        // the Y rows this lane updates, requested before the block loads and X gathers
-        float4 yo[BH];
-#pragma unroll
-        for (int h = 0; h < BH; h++) {
-            const int r = br * BH + h;
-            yo[h] = (valid && active && sub == 0 && r < m) ? *reinterpret_cast<const float4*>(y + (size_t)r * k + c)
-                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        for (int j0 = s; j0 < e; j0 += L) {
-            const int nb = min(L, e - j0);
-            __syncwarp(gmask);
-            if (lane < nb) {
-                s_col[gbase + lane] = __ldg(col + j0 + lane);
-#pragma unroll
-                for (int q = 0; q < BS; q++) s_val[(gbase + lane) * BS + q] = Val<V>::ld(data + (size_t)q * aligned + j0 + lane);
-            }
-            __syncwarp(gmask);
-            if (active) {
-                // U blocks of this sub-group at a time: their X rows are requested together.
-                // With 8 float4 lanes (k >= 32), U = 2 keeps the kernel at 58 registers,
-                // 4 CTAs per SM; U = 4 took 80 and ran 17 % slower on 3x3 blocks at k = 32
-                constexpr int U = (BW <= 3 && CW < 8) ? 4 : 2;
-                for (int t0 = sub; t0 < nb; t0 += S * U) {
-                    float4 xv[U][BW];
-#pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        const int t = t0 + u * S;
-                        const int bc = t < nb ? s_col[gbase + t] : 0;
-#pragma unroll
-                        for (int w = 0; w < BW; w++)
-                            xv[u][w] = (t < nb && bc + w < n)
-                                           ? __ldg(reinterpret_cast<const float4*>(x + (size_t)(bc + w) * k + c))
-                                           : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        const int t = t0 + u * S;
-                        if (t >= nb) break;
-                        const float* bv = s_val + (gbase + t) * BS;
-#pragma unroll
-                        for (int h = 0; h < BH; h++)
-#pragma unroll
-                            for (int w = 0; w < BW; w++) {
-                                const float a = bv[h * BW + w];
-                                acc[h].x += a * xv[u][w].x;
-                                acc[h].y += a * xv[u][w].y;
-                                acc[h].z += a * xv[u][w].z;
-                                acc[h].w += a * xv[u][w].w;
-                            }
-                    }
-                }
-            }
-        }
-        // sum the S sub-groups (lanes cw, cw + CW, ...)
-#pragma unroll
-        for (int h = 0; h < BH; h++) {
-#pragma unroll
-            for (int o = CW; o < L; o <<= 1) {
-                acc[h].x += __shfl_xor_sync(gmask, acc[h].x, o, L);
-                acc[h].y += __shfl_xor_sync(gmask, acc[h].y, o, L);
-                acc[h].z += __shfl_xor_sync(gmask, acc[h].z, o, L);
-                acc[h].w += __shfl_xor_sync(gmask, acc[h].w, o, L);
-            }
-        }
-        if (valid && active && sub == 0) {
+        float yv[BH];
+        auto begin_row = [&](int end) {
+            re = end;
 #pragma unroll
             for (int h = 0; h < BH; h++) {
-                const int r = br * BH + h;
-                if (r < m) {
-                    float4 o = yo[h];
-                    o.x += acc[h].x;
-                    o.y += acc[h].y;
-                    o.z += acc[h].z;
-                    o.w += acc[h].w;
-                    *reinterpret_cast<float4*>(y + (size_t)r * k + c) = o;
+                acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+                yv[h] = (writer && r * BH + h < m) ? yp[(size_t)h * k] : 0.0f;
+            }
+        };
+        const int end0 = __shfl_sync(0xffffffffu, rend, 0, GL);
+        if (r < r1) begin_row(end0);
+        while (__any_sync(0xffffffffu, r < r1)) {
+            // the blocks of this step: [j, min(j + 4 U, re)), all landed
+            const int jn = min(j + 4 * U, re);
+            bool need = j < re && jn > base + next * CH;
+            while (__any_sync(0xffffffffu, need)) {
+                __syncwarp();       // the slot about to be filled is no longer read
+                if (need) {
+                    issue(next + 2);
+                    asm volatile("cp.async.wait_group 2;\n" ::);
+                    next++;
+                    need = jn > base + next * CH;
+                }
+                __syncwarp();
+            }
+            const unsigned* bk[U];
+            float4 xv[U][BW];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int t = j + 4 * u + sub;
+                bk[u] = ring + ((t - base) & RM) * NW;
+                const unsigned off = t < re ? bk[u][Rec::xrow_word] : 0u;
+                const char* xp = xc + (size_t)off * 16;
+#pragma unroll
+                for (int w = 0; w < BW; w++) xv[u][w] = __ldg(reinterpret_cast<const float4*>(xp + w * kb));
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (j + 4 * u + sub >= re) continue;
+                float a[BS];
+                read_block<V, BS>(bk[u], a);
+#pragma unroll
+                for (int w = 0; w < BW; w++)
+#pragma unroll
+                    for (int h = 0; h < BH; h++) {
+                        acc[h].x += a[h * BW + w] * xv[u][w].x;
+                        acc[h].y += a[h * BW + w] * xv[u][w].y;
+                        acc[h].z += a[h * BW + w] * xv[u][w].z;
+                        acc[h].w += a[h * BW + w] * xv[u][w].w;
+                    }
+            }
+            j = jn;
+            const bool done = r < r1 && j == re;
+            if (__any_sync(0xffffffffu, done)) {
+                const bool up = lane & CW, up2 = lane & (2 * CW);
+                const int end = __shfl_sync(0xffffffffu, rend, min(r + 1 - r0, GL - 1), GL);
+                float out[BH];
+#pragma unroll
+                for (int h = 0; h < BH; h++) {
+                    float a = up ? acc[h].z : acc[h].x, b = up ? acc[h].w : acc[h].y;
+                    a += __shfl_xor_sync(0xffffffffu, up ? acc[h].x : acc[h].z, CW);
+                    b += __shfl_xor_sync(0xffffffffu, up ? acc[h].y : acc[h].w, CW);
+                    out[h] = (up2 ? b : a) + __shfl_xor_sync(0xffffffffu, up2 ? a : b, 2 * CW);
+                }
+                if (done) {
+#pragma unroll
+                    for (int h = 0; h < BH; h++)
+                        if (writer && r * BH + h < m) yp[(size_t)h * k] = yv[h] + out[h];
+                    r++;
+                    yp += (size_t)BH * k;
+                    if (r < r1) begin_row(end);
                 }
             }
         }
+        // the chunks issued ahead land before the ring is used again
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncwarp();
     }
 }
 
