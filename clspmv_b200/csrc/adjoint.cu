@@ -298,7 +298,7 @@ int Engine::build_adjoint(const cocktail_iif* mat)
     // --- transposed parts (built with rows and columns swapped) ---
     std::swap(width, height);
     std::swap(parts, adj_parts);
-    auto add_tdia = [&](const std::vector<int>& off, const float* data, int len, int valid_rows, int method) {
+    auto add_tdia = [&](const std::vector<int>& off, const float* data, int len, int valid_rows) {
         std::vector<int> off_t;
         std::vector<float> data_t;
         transpose_dia(height, len, off, data, valid_rows, off_t, data_t);
@@ -311,7 +311,7 @@ int Engine::build_adjoint(const cocktail_iif* mat)
         t.dia_length_aligned = len;
         t.dia_offsets = off_t.data();
         t.dia_data = data_t.data();
-        return add_dia(t, method);
+        return add_dia(t);
     };
     rc = CSP_OK;
     if (square && mat->ifusebdia) {
@@ -319,12 +319,12 @@ int Engine::build_adjoint(const cocktail_iif* mat)
         std::vector<int> off;
         for (int band = 0; band < b.bdia_band_num; band++)
             for (int k = b.bdia_bptr[band]; k < b.bdia_bptr[band + 1]; k++) off.push_back(b.bdia_offsets[band] + (k - b.bdia_bptr[band]));
-        rc = add_tdia(off, b.bdia_data, b.bdia_length_aligned, std::min(b.matinfo.height, b.bdia_length_aligned), 1);
+        rc = add_tdia(off, b.bdia_data, b.bdia_length_aligned, std::min(b.matinfo.height, b.bdia_length_aligned));
     }
     if (!rc && square && mat->ifusedia) {
         const dia_matrix_iif& d = mat->dia;
         std::vector<int> off(d.dia_offsets, d.dia_offsets + d.dia_num);
-        rc = add_tdia(off, d.dia_data, d.dia_length_aligned, std::min(d.matinfo.height, d.dia_length_aligned), 1);
+        rc = add_tdia(off, d.dia_data, d.dia_length_aligned, std::min(d.matinfo.height, d.dia_length_aligned));
     }
     std::swap(parts, adj_parts);
     std::swap(width, height);

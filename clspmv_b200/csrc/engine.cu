@@ -12,6 +12,7 @@
 #include <cuda_bf16.h>
 #include <stdio.h>
 #include <stdlib.h>
+#include <limits.h>
 #include <string.h>
 #include <algorithm>
 #include <cmath>
@@ -455,7 +456,29 @@ int Engine::add_sell(const sell_matrix_if& s, int method)
     return CSP_OK;
 }
 
-int Engine::add_dia(const dia_matrix_iif& d, int method)
+// Groups of at most dev::kDiaGroup diagonals, in stored order, with consecutive offsets
+// (dia_rows_kernel).
+int Engine::upload_dia_groups(Part& p, const std::vector<int>& off)
+{
+    std::vector<int2> groups;
+    for (size_t d = 0; d < off.size(); d++) {
+        const bool joins = !groups.empty() && groups.back().y < dev::kDiaGroup && off[d] != INT_MIN && off[d] - 1 == off[d - 1];
+        if (joins) groups.back().y++;
+        else groups.push_back(make_int2(off[d], 1));
+    }
+    p.ngroups = (int)groups.size();
+    if (groups.empty()) return CSP_OK;
+    p.off_min = *std::min_element(off.begin(), off.end());
+    p.off_max = *std::max_element(off.begin(), off.end());
+    int rc = alloc(reinterpret_cast<void**>(&p.dgroups), groups.size() * sizeof(int2));
+    if (rc) return rc;
+    CSP_CUDA(cudaMemcpy(p.dgroups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    return CSP_OK;
+}
+
+// Methods 0-3 of the reference (spmv_dia.cl) all run the four-row kernel, or a scalar one
+// where the diagonals are not aligned to four rows.
+int Engine::add_dia(const dia_matrix_iif& d)
 {
     const int len = d.dia_length_aligned;
     if (d.dia_num < 0 || len < 0 || (d.dia_num > 0 && (!d.dia_offsets || !d.dia_data)))
@@ -466,15 +489,19 @@ int Engine::add_dia(const dia_matrix_iif& d, int method)
     p.m = std::min(std::min(d.matinfo.height, height), len);
     p.k = d.dia_num;
     p.stride = len;
-    p.method = ((method == 1 || method == 3) && len % 4 == 0) ? 1 : 0;
+    p.method = len % 4 == 0 ? 1 : 0;
     const size_t n = (size_t)d.dia_num * len;
     int rc;
+    if (p.method == 1 && (rc = upload_dia_groups(p, std::vector<int>(d.dia_offsets, d.dia_offsets + d.dia_num)))) return rc;
     if ((rc = upload_int(&p.i0, d.dia_offsets, d.dia_num, d.dia_num)) || (rc = upload_val(&p.v, d.dia_data, n, n))) return rc;
     parts.push_back(p);
     return CSP_OK;
 }
 
-int Engine::add_bdia(const bdia_matrix_iif& b, int method)
+// Every BDIA method of the reference (spmv_cocktail.cpp:339-358: 0 nlvec, 1 staged, 2 staged
+// (g4), 3 v4_nlvec, 4 v4 staged) runs the four-row diagonal kernel over the bands' expanded
+// offsets; diagonals not aligned to four rows, the staged one.
+int Engine::add_bdia(const bdia_matrix_iif& b)
 {
     const int len = b.bdia_length_aligned;
     if (b.bdia_band_num < 0 || len < 0 || (b.bdia_band_num > 0 && (!b.bdia_offsets || !b.bdia_bptr || !b.bdia_data)))
@@ -482,25 +509,31 @@ int Engine::add_bdia(const bdia_matrix_iif& b, int method)
     Part p;
     p.kind = PART_BDIA;
     p.m = std::min(std::min(b.matinfo.height, height), len);
-    p.k = b.bdia_band_num;
     p.stride = len;
     const int ndia = b.bdia_band_num ? b.bdia_bptr[b.bdia_band_num] : 0;
     int maxw = 1;
     for (int i = 0; i < b.bdia_band_num; i++) maxw = std::max(maxw, b.bdia_bptr[i + 1] - b.bdia_bptr[i]);
     p.maxw = maxw;
-    // reference numbering (spmv_cocktail.cpp:339-358): 0 nlvec, 1 staged, 2 staged (g4),
-    // 3 v4_nlvec, 4 v4 staged
-    p.method = ((method == 0 || method == 3) && len % 4 == 0) ? 0 : 1;
-    if (maxw > 8000) p.method = 0;   // staged window would not fit in shared memory
-    if (p.method == 0 && len % 4 != 0) return set_error(CSP_EUNSUP, "BDIA part: band wider than 8000 with unaligned length");
+    p.method = len % 4 == 0 ? 1 : 0;
+    // the staged kernel's window would not fit in shared memory
+    if (p.method == 0 && maxw > 8000) return set_error(CSP_EUNSUP, "BDIA part: band wider than 8000 with unaligned length");
     for (int i = 0; i < b.bdia_band_num; i++)
         if (b.bdia_bptr[i + 1] < b.bdia_bptr[i] || b.bdia_bptr[0] != 0) return set_error(CSP_EINVAL, "BDIA part: bad band pointer");
     const size_t n = (size_t)ndia * len;
     int rc;
-    if ((rc = upload_int(&p.i0, b.bdia_offsets, b.bdia_band_num, b.bdia_band_num)) ||
-        (rc = upload_int(&p.i1, b.bdia_bptr, (size_t)b.bdia_band_num + 1, (size_t)b.bdia_band_num + 1)) ||
-        (rc = upload_val(&p.v, b.bdia_data, n, n)))
-        return rc;
+    if (p.method == 1) {
+        std::vector<int> off;
+        for (int i = 0; i < b.bdia_band_num; i++)
+            for (int k = b.bdia_bptr[i]; k < b.bdia_bptr[i + 1]; k++) off.push_back(b.bdia_offsets[i] + (k - b.bdia_bptr[i]));
+        p.k = ndia;
+        if ((rc = upload_dia_groups(p, off))) return rc;
+    } else {
+        p.k = b.bdia_band_num;
+        if ((rc = upload_int(&p.i0, b.bdia_offsets, b.bdia_band_num, b.bdia_band_num)) ||
+            (rc = upload_int(&p.i1, b.bdia_bptr, (size_t)b.bdia_band_num + 1, (size_t)b.bdia_band_num + 1)))
+            return rc;
+    }
+    if ((rc = upload_val(&p.v, b.bdia_data, n, n))) return rc;
     parts.push_back(p);
     return CSP_OK;
 }
@@ -853,23 +886,20 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
         if (p.method == 1) sell4_kernel<V><<<grid_for((p.m + 3) / 4, 256), 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m, p.stride);
         else sell1_kernel<V><<<grid_for(p.m, 256), 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m, p.stride);
         break;
-    case PART_DIA: {
+    case PART_DIA:
+    case PART_BDIA:
         if (p.m == 0) return;
-        const size_t sm = (size_t)std::max(p.k, 1) * sizeof(int);
-        if (p.method == 1) dia4_kernel<V><<<grid_for((p.m + 3) / 4, kDiaThreads), kDiaThreads, sm, st>>>(p.i0, v, x, y, p.m, n, p.k, p.stride);
-        else dia_kernel<V, 2><<<grid_for(p.m, kDiaThreads * 2), kDiaThreads, sm, st>>>(p.i0, v, x, y, p.m, n, p.k, p.stride);
-        break;
-    }
-    case PART_BDIA: {
-        if (p.m == 0) return;
-        if (p.method == 0) {
-            bdia4_kernel<V><<<grid_for((p.m + 3) / 4, kDiaThreads), kDiaThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.m, n, p.k, p.stride);
+        if (p.method == 1) {
+            dia_rows_kernel<V><<<grid_for((p.m + 3) / 4, kDiaRowsThreads), kDiaRowsThreads, 0, st>>>(
+                p.dgroups, v, x, y, y, p.m, n, p.ngroups, p.stride, p.off_min, p.off_max);
+        } else if (p.kind == PART_DIA) {
+            const size_t sm = (size_t)std::max(p.k, 1) * sizeof(int);
+            dia_kernel<V, 2><<<grid_for(p.m, kDiaThreads * 2), kDiaThreads, sm, st>>>(p.i0, v, x, y, p.m, n, p.k, p.stride);
         } else {
             const size_t sm = (size_t)(kDiaThreads * 4 + p.maxw) * sizeof(float);
             bdia_staged_kernel<V, 4><<<grid_for(p.m, kDiaThreads * 4), kDiaThreads, sm, st>>>(p.i0, p.i1, v, x, y, p.m, n, p.k, p.stride);
         }
         break;
-    }
     case PART_BELL: {
         if (p.nbr == 0) return;
         const unsigned g = grid_for(p.nbr, 256);
@@ -1135,8 +1165,8 @@ int Engine::init(const cocktail_iif* mat, const float* vec, const float* res, in
         if (flags & CSP_FLAG_ADJOINT) return set_error(CSP_EUNSUP, "adjoint with several right-hand sides");
     }
     // parts, in the reference's launch order
-    if (mat->ifusebdia && (rc = add_bdia(mat->bdia, mat->bdia_meth_num))) return rc;
-    if (mat->ifusedia && (rc = add_dia(mat->dia, mat->dia_meth_num))) return rc;
+    if (mat->ifusebdia && (rc = add_bdia(mat->bdia))) return rc;
+    if (mat->ifusedia && (rc = add_dia(mat->dia))) return rc;
     if (mat->ifusesbell && (rc = add_sbell(mat->sbell, mat->sbell_meth_num))) return rc;
     if (mat->ifusebell && (rc = add_bell(mat->bell, mat->bell_meth_num))) return rc;
     if (generic_bcsr) {

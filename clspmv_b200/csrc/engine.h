@@ -35,6 +35,9 @@ struct Part {
     int f4 = 0;       // BELL float4_aligned
     int bw = 0, bh = 0, nbr = 0;
     int maxw = 0;     // BDIA widest band
+    int2* dgroups = nullptr;        // DIA, BDIA: groups of consecutive offsets {first offset, diagonals}
+    int ngroups = 0;
+    int off_min = 0, off_max = 0;   // smallest and largest offset
     int group = 0;    // CSR sub-warp lanes per row
     int nblocks = 0;  // CSR adaptive row blocks
     bool records = false;  // generic BCSR, k % 4 == 0: v holds block records (kernels/spmm.cuh)
@@ -119,8 +122,9 @@ struct Engine {
     int add_xpanel(const int* rows, const int* cols, const float* vals, int nnz, bool from_csr);
     int add_ell(const ell_matrix_if& e, int method);
     int add_sell(const sell_matrix_if& s, int method);
-    int add_dia(const dia_matrix_iif& d, int method);
-    int add_bdia(const bdia_matrix_iif& b, int method);
+    int add_dia(const dia_matrix_iif& d);
+    int upload_dia_groups(Part& p, const std::vector<int>& off);
+    int add_bdia(const bdia_matrix_iif& b);
     int add_bell(const b4ell_matrix_if& b, int method);
     int add_sbell(const sbell_matrix_if& s, int method);
     int add_bcsr(const b4csr_matrix_if& b, int method);

@@ -17,6 +17,8 @@ template <> struct Val<float> {
     __device__ __forceinline__ static float ld(const float* p) { return __ldg(p); }
     // Four consecutive values; p must be 16-byte aligned.
     __device__ __forceinline__ static float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+    // The same from shared memory.
+    __device__ __forceinline__ static float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 };
 
 template <> struct Val<__nv_bfloat16> {
@@ -28,7 +30,11 @@ template <> struct Val<__nv_bfloat16> {
     // Four consecutive values; p must be 8-byte aligned.
     __device__ __forceinline__ static float4 ld4(const __nv_bfloat16* p)
     {
-        uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+        return widen(__ldg(reinterpret_cast<const uint2*>(p)));
+    }
+    __device__ __forceinline__ static float4 lds4(const __nv_bfloat16* p) { return widen(*reinterpret_cast<const uint2*>(p)); }
+    __device__ __forceinline__ static float4 widen(uint2 u)
+    {
         float4 f;
         f.x = __uint_as_float(u.x << 16);
         f.y = __uint_as_float(u.x & 0xffff0000u);
