@@ -840,6 +840,45 @@ static void launch_spmm(const Part& p, const float* x, float* y, int n, int k, b
     }
 }
 
+// Launches a kernel; `chained`: it may start before the previous kernel of the stream has
+// finished, up to its grid_dependency() (programmatic stream serialization).
+template <class... P, class... A>
+static void launch(void (*kernel)(P...), unsigned grid, int threads, bool chained, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // errors are read by enqueue_parts / iterate
+}
+
+// Parts whose kernels take the accumulated vector and the result apart (yout = yin + A x).
+static bool has_step(const Part& p)
+{
+    return (p.kind == PART_CSR && p.method == 2) || (p.kind == PART_ELL && p.method == 1) ||
+           ((p.kind == PART_DIA || p.kind == PART_BDIA) && p.method == 1);
+}
+
+template <class V>
+static void launch_step(const Part& p, const float* x, const float* yin, float* yout, int n, bool chained, cudaStream_t st)
+{
+    using namespace dev;
+    const V* v = static_cast<const V*>(p.v);
+    if (p.kind == PART_CSR)
+        launch(csr_adaptive_kernel<V>, p.nblocks, kAdaptThreads, chained, st, p.i0, p.i1, v, x, yin, yout, p.blocks, p.long_rows,
+               p.scratch_val, p.scratch_row);
+    else if (p.kind == PART_ELL)
+        launch(ell_rows_kernel<V>, grid_for((p.m + 3) / 4, 256), 256, chained, st, p.i1, v, x, yin, yout, p.m, p.k, p.stride);
+    else
+        launch(dia_rows_kernel<V>, grid_for((p.m + 3) / 4, kDiaRowsThreads), kDiaRowsThreads, chained, st, p.dgroups, v, x, yin, yout,
+               p.m, n, p.ngroups, p.stride, p.off_min, p.off_max);
+}
+
 template <class V>
 static void launch_part(const Part& p, const float* x, float* y, int n, cudaStream_t st)
 {
@@ -851,8 +890,7 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
         switch (p.method) {
         case 0: csr_vector_kernel<V, 32><<<grid_for((long long)p.m * 32, 256), 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
         case 1: csr_block_row_kernel<V, 128><<<p.m, 128, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
-        case 2: csr_adaptive_kernel<V><<<p.nblocks, kAdaptThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.blocks, p.long_rows,
-                                                                             p.scratch_val, p.scratch_row); break;
+        case 2: launch_step<V>(p, x, y, y, n, false, st); break;
         case 3: {
             const unsigned g = grid_for((long long)p.m * p.group, 256);
             switch (p.group) {
@@ -878,8 +916,8 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
     }
     case PART_ELL:
         if (p.m == 0) return;
-        if (p.method == 1) ell_kernel<V, 4><<<grid_for((p.m + 3) / 4, 256), 256, 0, st>>>(p.i1, v, x, y, p.m, p.k, p.stride);
-        else ell_kernel<V, 1><<<grid_for(p.m, 256), 256, 0, st>>>(p.i1, v, x, y, p.m, p.k, p.stride);
+        if (p.method == 1) launch_step<V>(p, x, y, y, n, false, st);
+        else ell_kernel<V><<<grid_for(p.m, 256), 256, 0, st>>>(p.i1, v, x, y, p.m, p.k, p.stride);
         break;
     case PART_SELL:
         if (p.m == 0) return;
@@ -890,8 +928,7 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
     case PART_BDIA:
         if (p.m == 0) return;
         if (p.method == 1) {
-            dia_rows_kernel<V><<<grid_for((p.m + 3) / 4, kDiaRowsThreads), kDiaRowsThreads, 0, st>>>(
-                p.dgroups, v, x, y, y, p.m, n, p.ngroups, p.stride, p.off_min, p.off_max);
+            launch_step<V>(p, x, y, y, n, false, st);
         } else if (p.kind == PART_DIA) {
             const size_t sm = (size_t)std::max(p.k, 1) * sizeof(int);
             dia_kernel<V, 2><<<grid_for(p.m, kDiaThreads * 2), kDiaThreads, sm, st>>>(p.i0, v, x, y, p.m, n, p.k, p.stride);
@@ -1029,11 +1066,33 @@ int Engine::spmv(int ntimes)
 // the next vector) on the device: `iterations` times y += A x; x = y.  With
 // CSP_FLAG_GRAPH, kIterChunk iterations are captured as one CUDA graph (and the
 // remainder as another), so a long loop costs one graph launch per chunk.
-int Engine::iterate_once(cudaStream_t st)
+//
+// After the first step x equals y, so where one part's kernel writes every row from a
+// separate input (d_z is set then), the steps alternate between d_z and d_x -- each
+// reads its whole input from one and writes the other -- and only the last one writes y and
+// copies it to x.  Those launches are chained: a step starts while the previous one runs
+// and has its part of the matrix in flight before it waits for it.  64 steps in a graph on
+// one B200: 511 x 517 Laplacian as DIA 339 us with a copy after every step (318 with the
+// present DIA kernel), 189 so; 600 x 600 as CSR (50 steps) 379 -> 254 us.
+int Engine::enqueue_steps(int steps, cudaStream_t st)
 {
-    int rc = enqueue_once(st);
-    if (rc) return rc;
-    CSP_CUDA(cudaMemcpyAsync(d_x, d_y, (size_t)height * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    if (steps > 1 && d_z) {
+        const float *x = d_x, *yin = d_y;
+        for (int i = 0; i < steps; i++) {
+            float* out = i == steps - 1 ? d_y : (x == d_z ? d_x : d_z);
+            if (bf16) launch_step<__nv_bfloat16>(parts[0], x, yin, out, width, i > 0, st);
+            else launch_step<float>(parts[0], x, yin, out, width, i > 0, st);
+            x = yin = out;
+        }
+        CSP_CUDA(cudaGetLastError());
+        CSP_CUDA(cudaMemcpyAsync(d_x, d_y, (size_t)height * sizeof(float), cudaMemcpyDeviceToDevice, st));
+        return CSP_OK;
+    }
+    for (int i = 0; i < steps; i++) {
+        int rc = enqueue_once(st);
+        if (rc) return rc;
+        CSP_CUDA(cudaMemcpyAsync(d_x, d_y, (size_t)height * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    }
     return CSP_OK;
 }
 
@@ -1044,11 +1103,7 @@ int Engine::iterate(int iterations)
     if (nrhs != 1) return set_error(CSP_EUNSUP, "iterate with several right-hand sides");
     cudaStream_t st = stream;
     if (!use_graph) {
-        for (int i = 0; i < iterations; i++) {
-            int rc = iterate_once(st);
-            if (rc) return rc;
-        }
-        return CSP_OK;
+        return enqueue_steps(iterations, st);
     }
     auto graph_of = [&](int n, cudaGraphExec_t* out) -> int {
         cudaGraphExec_t& ge = iter_graphs[n];
@@ -1056,8 +1111,7 @@ int Engine::iterate(int iterations)
             if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
             cudaGraph_t g;
             CSP_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            int rc = CSP_OK;
-            for (int i = 0; i < n && !rc; i++) rc = iterate_once(st);
+            int rc = enqueue_steps(n, st);
             cudaError_t e = cudaStreamEndCapture(st, &g);
             if (rc) { if (e == cudaSuccess) cudaGraphDestroy(g); return rc; }
             if (e != cudaSuccess) return cuda_error(e, "cudaStreamEndCapture");
@@ -1134,11 +1188,14 @@ int Engine::init_common(int w, int h, int nz, const float* vec, const float* res
     // y: padded to a multiple of 1024 like the reference (spmv_cocktail.cpp:234)
     x_len = pad_to(std::max(width, 1), 64) + 64;
     y_len = pad_to(std::max(height, 1), 1024);
+    // a square matrix's x has room for csp_iterate's second vector behind it (one allocation:
+    // a second one adds 0.1-0.3 ms to the set-up)
+    const size_t x_floats = (size_t)x_len * nrhs * (width == height && nrhs == 1 ? 2 : 1);
     int rc;
-    if ((rc = alloc(reinterpret_cast<void**>(&d_x), (size_t)x_len * nrhs * 4)) ||
+    if ((rc = alloc(reinterpret_cast<void**>(&d_x), x_floats * 4)) ||
         (rc = alloc(reinterpret_cast<void**>(&d_y), (size_t)y_len * nrhs * 4)))
         return rc;
-    CSP_CUDA(cudaMemset(d_x, 0, (size_t)x_len * nrhs * 4));
+    CSP_CUDA(cudaMemset(d_x, 0, x_floats * 4));
     CSP_CUDA(cudaMemset(d_y, 0, (size_t)y_len * nrhs * 4));
     if (vec && width) CSP_CUDA(cudaMemcpy(d_x, vec, (size_t)width * nrhs * 4, cudaMemcpyHostToDevice));
     if (res && height) CSP_CUDA(cudaMemcpy(d_y, res, (size_t)height * nrhs * 4, cudaMemcpyHostToDevice));
@@ -1180,6 +1237,8 @@ int Engine::init(const cocktail_iif* mat, const float* vec, const float* res, in
     if (mat->ifusecsr && (rc = add_csr(mat->csr, mat->csr_meth_num))) return rc;
     if (mat->ifusecoo && (rc = add_coo(mat->coo, mat->coo_meth_num))) return rc;
     if ((flags & CSP_FLAG_ADJOINT) && (rc = build_adjoint(mat))) return rc;
+    if (width == height && nrhs == 1 && parts.size() == 1 && has_step(parts[0]) && parts[0].m == height && height > 0)
+        d_z = d_x + x_len;   // csp_iterate
     CSP_CUDA(cudaDeviceSynchronize());
     return CSP_OK;
 }

@@ -78,6 +78,7 @@ struct Engine {
     cudaStream_t stream = nullptr;
     float* d_x = nullptr;
     float* d_y = nullptr;
+    float* d_z = nullptr;    // csp_iterate's second vector, where its steps alternate (enqueue_steps)
     int x_len = 0, y_len = 0;
     std::vector<Part> parts;
     std::vector<void*> allocations;
@@ -101,7 +102,7 @@ struct Engine {
     int init_bcsr(const bcsr_matrix_if* b, const float* vec, const float* res, int flags, int k);
     int spmv(int ntimes);
     int iterate(int iterations);
-    int iterate_once(cudaStream_t st);
+    int enqueue_steps(int steps, cudaStream_t st);
     int set_l2_window();
     int enqueue_once(cudaStream_t st);
     int enqueue_parts(const std::vector<Part>& ps, const float* x, float* y, int n, cudaStream_t st);

@@ -44,6 +44,18 @@ template <> struct Val<__nv_bfloat16> {
     }
 };
 
+// The point of a kernel after which it may touch what the kernel before it in the stream
+// reads or writes: x and y.  In a chain of launches with programmatic stream serialization
+// (csp_iterate) the part before it -- loads of the matrix -- overlaps the previous kernel;
+// in any other launch it returns at once.  The next kernel is let in only here, after the
+// previous one has completed, so at most two of the chain run at a time and no SM holds
+// lines of x from two steps ago.  x is read by plain loads in such kernels (it is written
+// within the life of a waiting kernel, which the read-only path does not allow).
+__device__ __forceinline__ void grid_dependency()
+{
+    asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 __device__ __forceinline__ int4 ld_int4(const int* p) { return __ldg(reinterpret_cast<const int4*>(p)); }
 __device__ __forceinline__ float ldx(const float* x, int i) { return __ldg(x + i); }
 __device__ __forceinline__ float4 ldx4(const float* x, int i) { return __ldg(reinterpret_cast<const float4*>(x + i)); }

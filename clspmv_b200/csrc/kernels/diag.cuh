@@ -64,19 +64,16 @@ __global__ void __launch_bounds__(kDiaThreads) dia_kernel(const int* __restrict_
 // matrix for some offset (omin .. omax) take guarded scalar loads of x.  x and y of any
 // 4-byte alignment are taken (the adjoint's vectors are the caller's).
 // Measured on one B200 (27 diagonals, before: a scalar guarded x load per entry, or for
-// BDIA x staged per band between two barriers): 160^3 FP32 BDIA 94.5 -> 82 us (6.0 TB/s),
-// 97^3 FP32 DIA 33.5 -> 22.8, 150^3 BF16 70 -> 53; 5 CTAs an SM with one group ahead and 3 with
-// three groups ahead are within 2 % of each other, 8 CTAs 8 % slower.
+// BDIA x staged per band between two barriers): 160^3 FP32 BDIA 94.5 -> 80.5 us (6.1 TB/s),
+// 97^3 FP32 DIA 33.5 -> 20.8, 150^3 BF16 70 -> 53.  FP32 also requests the next group's
+// window ahead (97^3: 22.8 us without) and does best at 3 CTAs an SM; BF16 keeps 5 CTAs
+// resident instead (53 us against 66).
 //
-// The first groups are requested before griddepcontrol.wait, so that in a chain of launches
-// with programmatic serialization (csp_iterate) they overlap the previous step; in any
-// other launch the wait returns at once.
+// The first groups are requested before grid_dependency(), so that they overlap the previous
+// step of csp_iterate.
 constexpr int kDiaRowsThreads = 256;
 constexpr int kDiaGroup = 3;   // 3 + 4 + (kDiaGroup - 1) floats: at most three vectors
 template <class V> struct DiaStages { static constexpr int n = sizeof(V) == 4 ? 2 : 4; };   // powers of two: the same bytes in flight
-
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 // acc += a[k] * x[S + k ..], the window v starting S floats before the group's first entry
 template <int S>
@@ -93,10 +90,11 @@ __device__ __forceinline__ void dia_fma(float4& acc, const float4 (&a)[kDiaGroup
 }
 
 template <class V>
-__global__ void __launch_bounds__(kDiaRowsThreads, 5) dia_rows_kernel(const int2* __restrict__ groups, const V* __restrict__ data,
+__global__ void __launch_bounds__(kDiaRowsThreads, sizeof(V) == 4 ? 3 : 5) dia_rows_kernel(const int2* __restrict__ groups, const V* __restrict__ data,
                                                                    const float* x, const float* yin, float* yout, int m, int n,
                                                                    int ng, int len, int omin, int omax)
 {
+    constexpr bool kAhead = sizeof(V) == 4;   // the next group's window is in flight
     constexpr int NS = DiaStages<V>::n, ES = 4 * sizeof(V);   // bytes of a thread's four values
     __shared__ __align__(16) unsigned char s_val[NS * kDiaGroup][kDiaRowsThreads * ES];
     const int rb = blockIdx.x * (kDiaRowsThreads * 4);
@@ -123,8 +121,7 @@ __global__ void __launch_bounds__(kDiaRowsThreads, 5) dia_rows_kernel(const int2
     };
 #pragma unroll
     for (int g = 0; g < NS - 1; g++) issue(g);
-    grid_dependency_wait();
-    grid_launch_dependents();
+    grid_dependency();
     const bool yvec = ((reinterpret_cast<uintptr_t>(yin) | reinterpret_cast<uintptr_t>(yout)) & 15) == 0 && r0 + 3 < m;
     float4 yo = make_float4(0.f, 0.f, 0.f, 0.f);
     if (yvec) {
@@ -139,13 +136,9 @@ __global__ void __launch_bounds__(kDiaRowsThreads, 5) dia_rows_kernel(const int2
     const float* xa = x - e;
     const bool interior = (long long)rb + omin - 3 >= 0 && (long long)rb + 4 * (kDiaRowsThreads - 1) + omax + 12 <= n;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int g = 0; g < ng; g++) {
-        const int2 gd = __ldg(groups + g);
-        const int off = gd.x, w = gd.y;
+    // the window of x of one group, s floats before its first entry
+    auto window = [&](int off, int w, int s, float (&v)[12]) {
         const int c = r0 + off;
-        issue(g + NS - 1);
-        float v[12];
-        const int s = (off + e) & 3;   // uniform: rows come in fours
         if (interior) {
             const float4* q = reinterpret_cast<const float4*>(xa + (c + e - s));
             const float4 v0 = q[0];
@@ -162,17 +155,35 @@ __global__ void __launch_bounds__(kDiaRowsThreads, 5) dia_rows_kernel(const int2
             for (int k = 0; k < kDiaGroup + 3; k++)
                 if (k < w + 3 && c + k >= 0 && c + k < n) v[k] = x[c + k];
         }
+    };
+    float v[12], vn[12];
+    int2 gd = ng ? __ldg(groups) : make_int2(0, 0);
+    int s = interior ? (gd.x + e) & 3 : 0;   // uniform: rows come in fours
+    if (kAhead && ng) window(gd.x, gd.y, s, v);
+    for (int g = 0; g < ng; g++) {
+        const int w = gd.y, sc = s;
+        if (!kAhead) window(gd.x, w, s, v);
+        issue(g + NS - 1);
+        if (g + 1 < ng) {
+            gd = __ldg(groups + g + 1);
+            s = interior ? (gd.x + e) & 3 : 0;
+            if (kAhead) window(gd.x, gd.y, s, vn);
+        }
         asm volatile("cp.async.wait_group %0;\n" ::"n"(NS - 1) : "memory");
         const unsigned char* src = own + (g & (NS - 1)) * (kDiaGroup * kDiaRowsThreads * ES);
         float4 a[kDiaGroup];
 #pragma unroll
         for (int k = 0; k < kDiaGroup; k++)
             if (k < w) a[k] = Val<V>::lds4(reinterpret_cast<const V*>(src + k * kDiaRowsThreads * ES));
-        switch (interior ? s : 0) {
+        switch (sc) {
         case 0: dia_fma<0>(acc, a, v, w); break;
         case 1: dia_fma<1>(acc, a, v, w); break;
         case 2: dia_fma<2>(acc, a, v, w); break;
         default: dia_fma<3>(acc, a, v, w); break;
+        }
+        if (kAhead) {
+#pragma unroll
+            for (int k = 0; k < 12; k++) v[k] = vn[k];
         }
     }
     if (yvec) {

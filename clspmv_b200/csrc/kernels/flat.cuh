@@ -128,9 +128,9 @@ __global__ void __launch_bounds__(THREADS) csr_block_row_kernel(const int* __res
 // {chunk index, -(long row id + 1), first entry, end entry}; chunk blocks come first
 // in the grid.
 //
-// A CTA issues every independent load of its block at once -- the 128-bit column
-// and value vectors (at most two per thread), the block's row pointers and its y
-// values -- then the x gathers, so a block costs two dependent memory round trips.
+// yout = yin + A x.  A CTA issues every independent load of its block at once -- the
+// 128-bit column and value vectors (at most two per thread) and the block's row pointers,
+// then the y values -- then the x gathers, so a block costs two dependent memory round trips.
 // Products go to shared memory; each row is reduced by a lane group sized to the
 // block's row count and written once (y = y + sum).  A chunk of a long row writes
 // its partial sum to a scratch slot; the CTA that finishes a row's last chunk (an
@@ -161,8 +161,9 @@ __device__ __forceinline__ void adaptive_rows(const int* s_rp, const float* prod
 
 template <class V>
 __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* __restrict__ rp, const int* __restrict__ col,
-                                                                     const V* __restrict__ val, const float* __restrict__ x,
-                                                                     float* __restrict__ y, const int4* __restrict__ blocks,
+                                                                     const V* __restrict__ val, const float* x,
+                                                                     const float* yin, float* yout,
+                                                                     const int4* __restrict__ blocks,
                                                                      const int4* __restrict__ long_rows,
                                                                      float* __restrict__ partial, int* __restrict__ arrivals)
 {
@@ -188,23 +189,24 @@ __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* 
         // nrows can equal the CTA width, so the end pointer (= e) is written separately
         if (tid < nrows) s_rp[tid] = __ldg(rp + r0 + tid) - s4;
         if (tid == 0) s_rp[nrows] = e - s4;
-        if (tid < nrows) s_y[tid] = y[r0 + tid];
     }
+    grid_dependency();
+    if (tid < (code > 0 ? nrows : 0)) s_y[tid] = yin[r0 + tid];
     // --- dependent x gathers; entries outside [s, e) contribute nothing ---
     float4 p0, p1;
     {
         const int j = s4 + 4 * v0;
-        p0.x = (j + 0 >= s && j + 0 < e) ? a0.x * ldx(x, c0.x) : 0.0f;
-        p0.y = (j + 1 >= s && j + 1 < e) ? a0.y * ldx(x, c0.y) : 0.0f;
-        p0.z = (j + 2 >= s && j + 2 < e) ? a0.z * ldx(x, c0.z) : 0.0f;
-        p0.w = (j + 3 >= s && j + 3 < e) ? a0.w * ldx(x, c0.w) : 0.0f;
+        p0.x = (j + 0 >= s && j + 0 < e) ? a0.x * x[c0.x] : 0.0f;
+        p0.y = (j + 1 >= s && j + 1 < e) ? a0.y * x[c0.y] : 0.0f;
+        p0.z = (j + 2 >= s && j + 2 < e) ? a0.z * x[c0.z] : 0.0f;
+        p0.w = (j + 3 >= s && j + 3 < e) ? a0.w * x[c0.w] : 0.0f;
     }
     {
         const int j = s4 + 4 * v1;
-        p1.x = (j + 0 >= s && j + 0 < e) ? a1.x * ldx(x, c1.x) : 0.0f;
-        p1.y = (j + 1 >= s && j + 1 < e) ? a1.y * ldx(x, c1.y) : 0.0f;
-        p1.z = (j + 2 >= s && j + 2 < e) ? a1.z * ldx(x, c1.z) : 0.0f;
-        p1.w = (j + 3 >= s && j + 3 < e) ? a1.w * ldx(x, c1.w) : 0.0f;
+        p1.x = (j + 0 >= s && j + 0 < e) ? a1.x * x[c1.x] : 0.0f;
+        p1.y = (j + 1 >= s && j + 1 < e) ? a1.y * x[c1.y] : 0.0f;
+        p1.z = (j + 2 >= s && j + 2 < e) ? a1.z * x[c1.z] : 0.0f;
+        p1.w = (j + 3 >= s && j + 3 < e) ? a1.w * x[c1.w] : 0.0f;
     }
     if (code < 0) {
         // one chunk of a long row: CTA-wide sum to a scratch slot
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* 
             __threadfence();
             float tot = 0.0f;
             for (int k = 0; k < lr.z; k++) tot += __ldcg(partial + lr.y + k);
-            y[lr.x] += tot;
+            yout[lr.x] = yin[lr.x] + tot;
             arrivals[-code - 1] = 0;
         }
         return;
@@ -231,12 +233,12 @@ __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* 
     if (v0 < nvec) reinterpret_cast<float4*>(prod)[v0] = p0;
     if (v1 < nvec) reinterpret_cast<float4*>(prod)[v1] = p1;
     __syncthreads();
-    if (nrows * 32 <= kAdaptThreads) adaptive_rows<32>(s_rp, prod, s_y, r0, nrows, y);
-    else if (nrows * 16 <= kAdaptThreads) adaptive_rows<16>(s_rp, prod, s_y, r0, nrows, y);
-    else if (nrows * 8 <= kAdaptThreads) adaptive_rows<8>(s_rp, prod, s_y, r0, nrows, y);
-    else if (nrows * 4 <= kAdaptThreads) adaptive_rows<4>(s_rp, prod, s_y, r0, nrows, y);
-    else if (nrows * 2 <= kAdaptThreads) adaptive_rows<2>(s_rp, prod, s_y, r0, nrows, y);
-    else adaptive_rows<1>(s_rp, prod, s_y, r0, nrows, y);
+    if (nrows * 32 <= kAdaptThreads) adaptive_rows<32>(s_rp, prod, s_y, r0, nrows, yout);
+    else if (nrows * 16 <= kAdaptThreads) adaptive_rows<16>(s_rp, prod, s_y, r0, nrows, yout);
+    else if (nrows * 8 <= kAdaptThreads) adaptive_rows<8>(s_rp, prod, s_y, r0, nrows, yout);
+    else if (nrows * 4 <= kAdaptThreads) adaptive_rows<4>(s_rp, prod, s_y, r0, nrows, yout);
+    else if (nrows * 2 <= kAdaptThreads) adaptive_rows<2>(s_rp, prod, s_y, r0, nrows, yout);
+    else adaptive_rows<1>(s_rp, prod, s_y, r0, nrows, yout);
 }
 
 // ---------------------------------------------------------------------------
@@ -394,39 +396,66 @@ __global__ void __launch_bounds__(256) coo_segment_kernel(const int* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// ELL, column-major (spmv_ell.cl gpu_ell / gpu_ell_v4).  ROWS consecutive rows per
-// thread; ROWS = 4 uses 128-bit loads (height_aligned is a multiple of 4).
+// ELL, column-major, one row per thread (spmv_ell.cl gpu_ell).
 // ---------------------------------------------------------------------------
-template <class V, int ROWS>
+template <class V>
 __global__ void __launch_bounds__(256) ell_kernel(const int* __restrict__ col, const V* __restrict__ val,
                                                   const float* __restrict__ x, float* __restrict__ y,
                                                   int m, int ell_num, int hal)
 {
-    const int r0 = (blockIdx.x * blockDim.x + threadIdx.x) * ROWS;
+    const int r0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (r0 >= m) return;
-    if (ROWS == 4) {
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int k = 0; k < ell_num; k++) {
-            const size_t j = (size_t)k * hal + r0;
-            const int4 c = ld_int4(col + j);
-            const float4 a = Val<V>::ld4(val + j);
-            acc.x += a.x * ldx(x, c.x);
-            acc.y += a.y * ldx(x, c.y);
-            acc.z += a.z * ldx(x, c.z);
-            acc.w += a.w * ldx(x, c.w);
-        }
-        y[r0] += acc.x;
-        if (r0 + 1 < m) y[r0 + 1] += acc.y;
-        if (r0 + 2 < m) y[r0 + 2] += acc.z;
-        if (r0 + 3 < m) y[r0 + 3] += acc.w;
-    } else {
-        float acc = 0.0f;
-        for (int k = 0; k < ell_num; k++) {
-            const size_t j = (size_t)k * hal + r0;
-            acc += Val<V>::ld(val + j) * ldx(x, __ldg(col + j));
-        }
-        y[r0] += acc;
+    float acc = 0.0f;
+    for (int k = 0; k < ell_num; k++) {
+        const size_t j = (size_t)k * hal + r0;
+        acc += Val<V>::ld(val + j) * ldx(x, __ldg(col + j));
     }
+    y[r0] += acc;
+}
+
+// ELL, four consecutive rows per thread with 128-bit loads (spmv_ell.cl gpu_ell_v4;
+// height_aligned is a multiple of 4): yout = yin + A x.  The columns and values of
+// kEllAhead slots are requested together, the first ones before grid_dependency().
+constexpr int kEllAhead = 5;
+
+template <class V>
+__global__ void __launch_bounds__(256) ell_rows_kernel(const int* __restrict__ col, const V* __restrict__ val, const float* x,
+                                                       const float* yin, float* yout, int m, int ell_num, int hal)
+{
+    const int r0 = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (r0 >= m) return;
+    int4 c[kEllAhead];
+    float4 a[kEllAhead];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < kEllAhead; u++)
+            if (k0 + u < ell_num) {
+                const size_t j = (size_t)(k0 + u) * hal + r0;
+                c[u] = ld_int4(col + j);
+                a[u] = Val<V>::ld4(val + j);
+            }
+    };
+    fetch(0);
+    grid_dependency();
+    float yo[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) yo[q] = r0 + q < m ? yin[r0 + q] : 0.0f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < ell_num; k += kEllAhead) {
+        if (k) fetch(k);
+#pragma unroll
+        for (int u = 0; u < kEllAhead; u++) {
+            if (k + u >= ell_num) break;
+            acc.x += a[u].x * x[c[u].x];
+            acc.y += a[u].y * x[c[u].y];
+            acc.z += a[u].z * x[c[u].z];
+            acc.w += a[u].w * x[c[u].w];
+        }
+    }
+    yout[r0] = yo[0] + acc.x;
+    if (r0 + 1 < m) yout[r0 + 1] = yo[1] + acc.y;
+    if (r0 + 2 < m) yout[r0 + 2] = yo[2] + acc.z;
+    if (r0 + 3 < m) yout[r0 + 3] = yo[3] + acc.w;
 }
 
 // ---------------------------------------------------------------------------
