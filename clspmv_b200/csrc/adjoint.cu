@@ -20,6 +20,7 @@
 #include "csp/clspmv.h"
 #include "internal.h"
 #include "engine.h"
+#include "launch.h"
 #include "kernels/adjoint.cuh"
 
 namespace csp {
@@ -462,7 +463,7 @@ int Engine::build_adjoint(const cocktail_iif* mat)
     return CSP_OK;
 }
 
-int Engine::launch_abar(const float* ybar, float* abar, int* prow, int* pcol, cudaStream_t st)
+int Engine::launch_abar(const float* ybar, float* abar, int* prow, int* pcol, bool beside, cudaStream_t st)
 {
     using namespace dev;
     for (const Seg& s : segs) {
@@ -475,12 +476,12 @@ int Engine::launch_abar(const float* ybar, float* abar, int* prow, int* pcol, cu
         case SEG_DIA:
             if (a && s.p1 % 4 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0) {
                 const unsigned g4 = (unsigned)((s.p1 / 4 + 255) / 256);
-                abar_dia4_kernel<<<g4, 256, (size_t)s.p0 * sizeof(int), st>>>(s.a0, s.p0, s.p1, s.p2, width, ybar, d_x, a);
+                launch_chained(abar_dia4_kernel, g4, 256, (size_t)s.p0 * sizeof(int), st, s.a0, s.p0, s.p1, s.p2, width, ybar, d_x, a, beside);
             } else {
                 abar_dia_kernel<<<g, 256, 0, st>>>(s.a0, s.p0, s.p1, s.p2, width, ybar, d_x, a, pr, pc);
             }
             break;
-        case SEG_LIST: abar_list_kernel<<<g, 256, 0, st>>>(s.a0, s.a1, s.count, ybar, d_x, a, pr, pc); break;
+        case SEG_LIST: launch_chained(abar_list_kernel, g, 256, 0, st, s.a0, s.a1, s.count, ybar, d_x, a, pr, pc, beside); break;
         case SEG_GBCSR:
             abar_gbcsr_kernel<<<g, 256, 0, st>>>(s.a0, s.a1, s.p0, s.p1, s.p2 >> 4, s.p2 & 15, height, width, ybar, d_x, a,
                                                  pr, pc);
@@ -493,6 +494,7 @@ int Engine::launch_abar(const float* ybar, float* abar, int* prow, int* pcol, cu
         }
         default: break;
         }
+        beside = false;
     }
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CSP_OK : cuda_error(e, "adjoint value gradient");
@@ -511,11 +513,20 @@ int csp_spmv_adjoint(csp_handle* h, const float* d_ybar, float* d_xbar, float* d
     if (!e.adjoint) return set_error(CSP_EINVAL, "handle was not built with CSP_FLAG_ADJOINT");
     if (!d_ybar) return set_error(CSP_EINVAL, "null ybar");
     if (d_abar && e.abar_blocks) return set_error(CSP_EUNSUP, "value gradients of this handle's parts are not provided");
+    // the gradients' first kernel may run beside the transposed product's last one where that
+    // is a single launch that calls grid_dependency() first, and the results do not overlap
+    bool beside = false;
     if (d_xbar) {
         int rc = e.enqueue_parts(e.adj_parts, d_ybar, d_xbar, e.height, e.stream);
         if (rc) return rc;
+        const uintptr_t x0 = reinterpret_cast<uintptr_t>(d_xbar), x1 = x0 + (size_t)e.width * 4;
+        const uintptr_t y0 = reinterpret_cast<uintptr_t>(d_ybar), y1 = y0 + (size_t)e.height * 4;
+        const uintptr_t a0 = reinterpret_cast<uintptr_t>(d_abar), a1 = a0 + e.abar_total * 4;
+        const uintptr_t v0 = reinterpret_cast<uintptr_t>(e.d_x), v1 = v0 + (size_t)e.width * 4;
+        const bool apart = (x1 <= y0 || y1 <= x0) && (x1 <= a0 || a1 <= x0) && (x1 <= v0 || v1 <= x0) && (a1 <= y0 || y1 <= a0);
+        beside = d_abar && apart && csp::step_parts(e.adj_parts);
     }
-    if (d_abar) return e.launch_abar(d_ybar, d_abar, nullptr, nullptr, e.stream);
+    if (d_abar) return e.launch_abar(d_ybar, d_abar, nullptr, nullptr, beside, e.stream);
     return CSP_OK;
 }
 
@@ -532,7 +543,7 @@ int csp_adjoint_pattern(csp_handle* h, int* d_rows, int* d_cols)
     if (!h || !d_rows || !d_cols) return set_error(CSP_EINVAL, "null argument");
     if (!h->eng.adjoint) return set_error(CSP_EINVAL, "handle was not built with CSP_FLAG_ADJOINT");
     if (h->eng.abar_blocks) return set_error(CSP_EUNSUP, "value gradients of this handle's parts are not provided");
-    return h->eng.launch_abar(nullptr, nullptr, d_rows, d_cols, h->eng.stream);
+    return h->eng.launch_abar(nullptr, nullptr, d_rows, d_cols, false, h->eng.stream);
 }
 
 }  // extern "C"

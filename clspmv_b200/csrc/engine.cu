@@ -22,6 +22,7 @@
 #include "csp/clspmv.h"
 #include "internal.h"
 #include "engine.h"
+#include "launch.h"
 #include "kernels/flat.cuh"
 #include "kernels/diag.cuh"
 #include "kernels/block.cuh"
@@ -806,8 +807,8 @@ static void launch_spmm(const Part& p, const float* x, float* y, int n, int k, b
         const int wave = 148 * Sh::ctas * Sh::warps * Sh::groups;                                                                \
         const int rows = std::min(Sh::max_rows, (p.nbr + wave - 1) / wave);                                                      \
         const long long ng = ((long long)p.nbr + rows - 1) / rows;                                                               \
-        bcsr_spmm_stream_kernel<V, BH, BW, C, K><<<grid_for(ng * Sh::GL, Sh::threads), Sh::threads, 0, st>>>(                    \
-            p.i0, rec, x, y, p.nbr, p.m, k, rows);                                                                               \
+        launch_chained(bcsr_spmm_stream_kernel<V, BH, BW, C, K>, grid_for(ng * Sh::GL, Sh::threads), Sh::threads, 0, st,         \
+                       p.i0, rec, x, y, p.nbr, p.m, k, rows);                                                                    \
     } while (0)
 #define CSP_GB4(BH, BW)                                                                                                          \
     do {                                                                                                                         \
@@ -844,23 +845,6 @@ static void launch_spmm(const Part& p, const float* x, float* y, int n, int k, b
     }
 }
 
-// Launches a kernel; `chained`: it may start before the previous kernel of the stream has
-// finished, up to its grid_dependency() (programmatic stream serialization).
-template <class... P, class... A>
-static void launch(void (*kernel)(P...), unsigned grid, int threads, bool chained, cudaStream_t st, A... args)
-{
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = chained ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // errors are read by enqueue_parts / iterate
-}
-
 // Parts whose kernels take the accumulated vector and the result apart (yout = yin + A x).
 static bool has_step(const Part& p)
 {
@@ -868,19 +852,21 @@ static bool has_step(const Part& p)
            ((p.kind == PART_DIA || p.kind == PART_BDIA) && p.method == 1);
 }
 
+bool step_parts(const std::vector<Part>& parts) { return !parts.empty() && has_step(parts.back()) && parts.back().m > 0; }
+
 template <class V>
-static void launch_step(const Part& p, const float* x, const float* yin, float* yout, int n, bool chained, cudaStream_t st)
+static void launch_step(const Part& p, const float* x, const float* yin, float* yout, int n, cudaStream_t st)
 {
     using namespace dev;
     const V* v = static_cast<const V*>(p.v);
     if (p.kind == PART_CSR)
-        launch(csr_adaptive_kernel<V>, p.nblocks, kAdaptThreads, chained, st, p.i0, p.i1, v, x, yin, yout, p.blocks, p.long_rows,
+        launch_chained(csr_adaptive_kernel<V>, p.nblocks, kAdaptThreads, 0, st, p.i0, p.i1, v, x, yin, yout, p.blocks, p.long_rows,
                p.scratch_val, p.scratch_row);
     else if (p.kind == PART_ELL)
-        launch(ell_rows_kernel<V>, grid_for((p.m + 3) / 4, 256), 256, chained, st, p.i1, v, x, yin, yout, p.m, p.k, p.stride);
+        launch_chained(ell_rows_kernel<V>, grid_for((p.m + 3) / 4, 256), 256, 0, st, p.i1, v, x, yin, yout, p.m, p.k, p.stride);
     else
-        launch(dia_rows_kernel<V>, grid_for((p.m + 3) / 4, kDiaRowsThreads), kDiaRowsThreads, chained, st, p.dgroups, v, x, yin, yout,
-               p.m, n, p.ngroups, p.stride, p.off_min, p.off_max);
+        launch_chained(dia_rows_kernel<V>, grid_for((p.m + 3) / 4, kDiaRowsThreads), kDiaRowsThreads, 0, st, p.dgroups, v, x, yin,
+                       yout, p.m, n, p.ngroups, p.stride, p.off_min, p.off_max);
 }
 
 template <class V>
@@ -892,17 +878,17 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
     case PART_CSR: {
         if (p.m == 0) return;
         switch (p.method) {
-        case 0: csr_vector_kernel<V, 32><<<grid_for((long long)p.m * 32, 256), 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
+        case 0: launch_chained(csr_vector_kernel<V, 32>, grid_for((long long)p.m * 32, 256), 256, 0, st, p.i0, p.i1, v, x, y, p.m); break;
         case 1: csr_block_row_kernel<V, 128><<<p.m, 128, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
-        case 2: launch_step<V>(p, x, y, y, n, false, st); break;
+        case 2: launch_step<V>(p, x, y, y, n, st); break;
         case 3: {
             const unsigned g = grid_for((long long)p.m * p.group, 256);
             switch (p.group) {
-            case 2: csr_vector_kernel<V, 2><<<g, 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
-            case 4: csr_vector_kernel<V, 4><<<g, 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
-            case 8: csr_vector_kernel<V, 8><<<g, 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
-            case 16: csr_vector_kernel<V, 16><<<g, 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
-            default: csr_vector_kernel<V, 32><<<g, 256, 0, st>>>(p.i0, p.i1, v, x, y, p.m); break;
+            case 2: launch_chained(csr_vector_kernel<V, 2>, g, 256, 0, st, p.i0, p.i1, v, x, y, p.m); break;
+            case 4: launch_chained(csr_vector_kernel<V, 4>, g, 256, 0, st, p.i0, p.i1, v, x, y, p.m); break;
+            case 8: launch_chained(csr_vector_kernel<V, 8>, g, 256, 0, st, p.i0, p.i1, v, x, y, p.m); break;
+            case 16: launch_chained(csr_vector_kernel<V, 16>, g, 256, 0, st, p.i0, p.i1, v, x, y, p.m); break;
+            default: launch_chained(csr_vector_kernel<V, 32>, g, 256, 0, st, p.i0, p.i1, v, x, y, p.m); break;
             }
             break;
         }
@@ -913,14 +899,13 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
         break;
     }
     case PART_COO: {
-        coo_segment_kernel<V><<<grid_for((long long)p.nwarps * 32, 256), 256, 0, st>>>(p.i0, p.i1, v, x, y, p.npad, p.nwarps,
-                                                                                      p.span_head, p.spans, p.scratch_row,
-                                                                                      p.scratch_val);
+        launch_chained(coo_segment_kernel<V>, grid_for((long long)p.nwarps * 32, 256), 256, 0, st, p.i0, p.i1, v, x, y, p.npad, p.nwarps,
+                       p.span_head, p.spans, p.scratch_row, p.scratch_val);
         break;
     }
     case PART_ELL:
         if (p.m == 0) return;
-        if (p.method == 1) launch_step<V>(p, x, y, y, n, false, st);
+        if (p.method == 1) launch_step<V>(p, x, y, y, n, st);
         else ell_kernel<V><<<grid_for(p.m, 256), 256, 0, st>>>(p.i1, v, x, y, p.m, p.k, p.stride);
         break;
     case PART_SELL:
@@ -932,7 +917,7 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
     case PART_BDIA:
         if (p.m == 0) return;
         if (p.method == 1) {
-            launch_step<V>(p, x, y, y, n, false, st);
+            launch_step<V>(p, x, y, y, n, st);
         } else if (p.kind == PART_DIA) {
             const size_t sm = (size_t)std::max(p.k, 1) * sizeof(int);
             dia_kernel<V, 2><<<grid_for(p.m, kDiaThreads * 2), kDiaThreads, sm, st>>>(p.i0, v, x, y, p.m, n, p.k, p.stride);
@@ -983,18 +968,17 @@ static void launch_part(const Part& p, const float* x, float* y, int n, cudaStre
         break;
     }
     case PART_XPANEL: {
-        dev::xpanel_kernel<V><<<p.ncta, kXpThreads, p.smem, st>>>(
-            p.tile0, p.ntiles, p.npanels, p.i0, p.lcol, v, x, n, p.panel_w, p.partial, y);
+        launch_chained(xpanel_kernel<V>, p.ncta, kXpThreads, p.smem, st, p.tile0, p.ntiles, p.npanels, p.i0, p.lcol, v, x, n, p.panel_w, p.partial, y);
         // at least one CTA even when every row has one run: the launch count stays fixed
         const long long mthreads = (long long)grid_for(p.nrun_rows, 256) * 256 + (long long)p.nlong * kXpMergeLanes;
-        xpanel_merge_kernel<<<grid_for(std::max(mthreads, 1LL), 256), 256, 0, st>>>(p.run_ptr, p.run_rows, p.nrun_rows, p.long_list,
-                                                                     p.nlong, p.partial, y);
+        launch_chained(xpanel_merge_kernel, grid_for(std::max(mthreads, 1LL), 256), 256, 0, st, p.run_ptr, p.run_rows, p.nrun_rows,
+                       p.long_list, p.nlong, p.partial, y);
         break;
     }
     case PART_GBCSR: {
         if (p.nbr == 0) return;
         if (p.nblocks > 0) {
-#define CSP_GBA(BH, BW) bcsr_adaptive_kernel<V, BH, BW><<<p.nblocks, kGbThreads, 0, st>>>(p.i0, p.i1, v, x, y, p.blocks, p.lcol, p.stride, p.m, n)
+#define CSP_GBA(BH, BW) launch_chained(bcsr_adaptive_kernel<V, BH, BW>, p.nblocks, kGbThreads, 0, st, p.i0, p.i1, v, x, y, p.blocks, p.lcol, p.stride, p.m, n)
             switch (p.bh * 10 + p.bw) {
             case 11: CSP_GBA(1, 1); break; case 22: CSP_GBA(2, 2); break; case 33: CSP_GBA(3, 3); break;
             case 44: CSP_GBA(4, 4); break;
@@ -1074,8 +1058,8 @@ int Engine::spmv(int ntimes)
 // After the first step x equals y, so where one part's kernel writes every row from a
 // separate input (d_z is set then), the steps alternate between d_z and d_x -- each
 // reads its whole input from one and writes the other -- and only the last one writes y and
-// copies it to x.  Those launches are chained: a step starts while the previous one runs
-// and has its part of the matrix in flight before it waits for it.  64 steps in a graph on
+// copies it to x.  The launches are chained (launch.h): a step starts while the previous one
+// runs and has its part of the matrix in flight before it waits for it.  64 steps in a graph on
 // one B200: 511 x 517 Laplacian as DIA 339 us with a copy after every step (318 with the
 // present DIA kernel), 189 so; 600 x 600 as CSR (50 steps) 379 -> 254 us.
 int Engine::enqueue_steps(int steps, cudaStream_t st)
@@ -1084,8 +1068,8 @@ int Engine::enqueue_steps(int steps, cudaStream_t st)
         const float *x = d_x, *yin = d_y;
         for (int i = 0; i < steps; i++) {
             float* out = i == steps - 1 ? d_y : (x == d_z ? d_x : d_z);
-            if (bf16) launch_step<__nv_bfloat16>(parts[0], x, yin, out, width, i > 0, st);
-            else launch_step<float>(parts[0], x, yin, out, width, i > 0, st);
+            if (bf16) launch_step<__nv_bfloat16>(parts[0], x, yin, out, width, st);
+            else launch_step<float>(parts[0], x, yin, out, width, st);
             x = yin = out;
         }
         CSP_CUDA(cudaGetLastError());

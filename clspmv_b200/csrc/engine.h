@@ -111,7 +111,7 @@ struct Engine {
     int gbcsr_segment(const bcsr_matrix_if& b, Seg& s);
     int add_transposed_csr(std::vector<Entry>& e);
     int add_slot_list(Seg& s, const std::vector<int>& rows, const std::vector<int>& cols);
-    int launch_abar(const float* ybar, float* abar, int* prow, int* pcol, cudaStream_t st);
+    int launch_abar(const float* ybar, float* abar, int* prow, int* pcol, bool beside, cudaStream_t st);
     int launches_per_spmv() const;
 
     int alloc(void** p, size_t bytes);
@@ -134,6 +134,10 @@ struct Engine {
 };
 
 int cuda_error(cudaError_t e, const char* what);
+
+// Whether the last of these parts runs as one launch of a kernel whose grid_dependency()
+// comes before it lets the next launch in.
+bool step_parts(const std::vector<Part>& parts);
 
 // CSR adaptive work blocks (see csr_adaptive_kernel) of rows [0, m) of row pointer rp;
 // nslots = long-row chunk partial slots.

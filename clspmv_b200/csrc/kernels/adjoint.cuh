@@ -11,16 +11,29 @@
 namespace csp {
 namespace dev {
 
-__device__ __forceinline__ void put_slot(size_t i, int row, int col, const float* __restrict__ ybar,
-                                         const float* __restrict__ x, float* __restrict__ abar,
+__device__ __forceinline__ void put_slot(size_t i, int row, int col, const float* ybar,
+                                         const float* x, float* __restrict__ abar,
                                          int* __restrict__ prow, int* __restrict__ pcol)
 {
     if (prow) {
         prow[i] = row;
         pcol[i] = row < 0 ? -1 : col;
     } else {
-        abar[i] = row < 0 ? 0.0f : __ldg(ybar + row) * __ldg(x + col);
+        abar[i] = row < 0 ? 0.0f : ybar[row] * x[col];
     }
+}
+
+// Launches right behind the transposed product of the same call (`beside`): that kernel lets
+// them in only once everything before it has completed, and they touch nothing it writes,
+// so they run beside its tail and wait for it at their end (the next operation of the
+// stream then follows both).  Otherwise they wait first.
+__device__ __forceinline__ void gradient_begin(bool beside)
+{
+    if (!beside) grid_dependency();
+}
+__device__ __forceinline__ void gradient_end(bool beside)
+{
+    if (beside) grid_dependency();
 }
 
 // DIA-layout slots (also BDIA, whose slots carry per-slot offsets): slot (d, r)
@@ -46,17 +59,21 @@ __global__ void __launch_bounds__(256) abar_dia_kernel(const int* __restrict__ o
 // the host) and x is the handle's padded x; the offsets (nd of them) are staged in
 // shared memory.
 __global__ void __launch_bounds__(256) abar_dia4_kernel(const int* __restrict__ off, int nd, int len, int m, int n,
-                                                        const float* __restrict__ ybar, const float* __restrict__ x,
-                                                        float* __restrict__ abar)
+                                                        const float* ybar, const float* x,
+                                                        float* __restrict__ abar, bool beside)
 {
     extern __shared__ int s_off[];
     for (int i = threadIdx.x; i < nd; i += blockDim.x) s_off[i] = __ldg(off + i);
     __syncthreads();
+    gradient_begin(beside);
     const int r = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (r >= len) return;
+    if (r >= len) {
+        gradient_end(beside);
+        return;
+    }
     float yb[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) yb[q] = r + q < m ? __ldg(ybar + r + q) : 0.0f;
+    for (int q = 0; q < 4; q++) yb[q] = r + q < m ? ybar[r + q] : 0.0f;
     for (int d = 0; d < nd; d++) {
         const int base = r + s_off[d];
         float xv[4];
@@ -64,7 +81,7 @@ __global__ void __launch_bounds__(256) abar_dia4_kernel(const int* __restrict__ 
             // x[base .. base+3] from the two aligned float4s around it (x is 16-byte
             // aligned and zero-padded by at least 64 entries past n)
             const int b4 = base & ~3;
-            const float4 lo = ldx4(x, b4), hi = ldx4(x, b4 + 4);
+            const float4 lo = *reinterpret_cast<const float4*>(x + b4), hi = *reinterpret_cast<const float4*>(x + b4 + 4);
             switch (base - b4) {
             case 0: xv[0] = lo.x; xv[1] = lo.y; xv[2] = lo.z; xv[3] = lo.w; break;
             case 1: xv[0] = lo.y; xv[1] = lo.z; xv[2] = lo.w; xv[3] = hi.x; break;
@@ -73,23 +90,26 @@ __global__ void __launch_bounds__(256) abar_dia4_kernel(const int* __restrict__ 
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < 4; q++) xv[q] = (base + q >= 0 && base + q < n) ? __ldg(x + base + q) : 0.0f;
+            for (int q = 0; q < 4; q++) xv[q] = (base + q >= 0 && base + q < n) ? x[base + q] : 0.0f;
         }
         __stcs(reinterpret_cast<float4*>(abar + (size_t)d * len + r),
                make_float4(yb[0] * xv[0], yb[1] * xv[1], yb[2] * xv[2], yb[3] * xv[3]));
     }
+    gradient_end(beside);
 }
 
 // Slot lists with explicit row ids (COO; CSR with its row-id array; the block layouts'
 // slot maps, row -1 on padding slots).
 __global__ void __launch_bounds__(256) abar_list_kernel(const int* __restrict__ rows, const int* __restrict__ cols,
-                                                        size_t nslots, const float* __restrict__ ybar,
-                                                        const float* __restrict__ x, float* __restrict__ abar,
-                                                        int* __restrict__ prow, int* __restrict__ pcol)
+                                                        size_t nslots, const float* ybar,
+                                                        const float* x, float* __restrict__ abar,
+                                                        int* __restrict__ prow, int* __restrict__ pcol, bool beside)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nslots) return;
-    put_slot(i, __ldg(rows + i), __ldg(cols + i), ybar, x, abar, prow, pcol);
+    const int r = i < nslots ? __ldg(rows + i) : -1, c = i < nslots ? __ldg(cols + i) : 0;
+    gradient_begin(beside);
+    if (i < nslots) put_slot(i, r, c, ybar, x, abar, prow, pcol);
+    gradient_end(beside);
 }
 
 // Generic BCSR slots data[e * aligned + j]: element e of block j couples row

@@ -190,7 +190,7 @@ __device__ __forceinline__ void gb_rows(const int* s_rp, const float* prod, cons
 
 template <class V, int BH, int BW>
 __global__ void __launch_bounds__(kGbThreads) bcsr_adaptive_kernel(const int* __restrict__ rp, const int* __restrict__ col,
-                                                                   const V* __restrict__ data, const float* __restrict__ x,
+                                                                   const V* __restrict__ data, const float* x,
                                                                    float* __restrict__ y, const int4* __restrict__ work,
                                                                    const unsigned short* __restrict__ tgt, int aligned, int m,
                                                                    int n)
@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(kGbThreads) bcsr_adaptive_kernel(const int* __
     // does not wait on DRAM
     if (tid < nrows) s_rp[tid] = __ldg(rp + br0 + tid) - s;
     if (tid == 0) s_rp[nrows] = cnt;
+    grid_dependency();
     for (int i = tid; i < nrows * BH; i += kGbThreads)
         if (br0 * BH + i < m) s_y[i] = y[br0 * BH + i];
     if (act) {
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kGbThreads) bcsr_adaptive_kernel(const int* __
             const bool in = tq[q] != 0xffff;
             float xv[BW];
 #pragma unroll
-            for (int w = 0; w < BW; w++) xv[w] = (in && cc[q] + w < n) ? __ldg(x + cc[q] + w) : 0.0f;
+            for (int w = 0; w < BW; w++) xv[w] = (in && cc[q] + w < n) ? x[cc[q] + w] : 0.0f;
 #pragma unroll
             for (int h = 0; h < BH; h++) {
                 float t = 0.0f;

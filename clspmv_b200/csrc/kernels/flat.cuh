@@ -64,19 +64,19 @@ __global__ void __launch_bounds__(256) csr_scalar4_kernel(const int* __restrict_
 // aligned vector covering e-1 is always in bounds).
 template <class V, int G>
 __device__ __forceinline__ float segment_dot(const int* __restrict__ col, const V* __restrict__ val,
-                                             const float* __restrict__ x, int s, int e, int lane)
+                                             const float* x, int s, int e, int lane)
 {
     float acc = 0.0f;
     for (int j = (s & ~3) + 4 * lane; j < e; j += 4 * G) {
         const int4 c = ld_int4(col + j);
         const float4 v = Val<V>::ld4(val + j);
         if (j >= s && j + 3 < e) {
-            acc += v.x * ldx(x, c.x) + v.y * ldx(x, c.y) + v.z * ldx(x, c.z) + v.w * ldx(x, c.w);
+            acc += v.x * x[c.x] + v.y * x[c.y] + v.z * x[c.z] + v.w * x[c.w];
         } else {
-            if (j + 0 >= s && j + 0 < e) acc += v.x * ldx(x, c.x);
-            if (j + 1 >= s && j + 1 < e) acc += v.y * ldx(x, c.y);
-            if (j + 2 >= s && j + 2 < e) acc += v.z * ldx(x, c.z);
-            if (j + 3 >= s && j + 3 < e) acc += v.w * ldx(x, c.w);
+            if (j + 0 >= s && j + 0 < e) acc += v.x * x[c.x];
+            if (j + 1 >= s && j + 1 < e) acc += v.y * x[c.y];
+            if (j + 2 >= s && j + 2 < e) acc += v.z * x[c.z];
+            if (j + 3 >= s && j + 3 < e) acc += v.w * x[c.w];
         }
     }
     return acc;
@@ -90,7 +90,7 @@ __device__ __forceinline__ float segment_dot(const int* __restrict__ col, const 
 // ---------------------------------------------------------------------------
 template <class V, int G>
 __global__ void __launch_bounds__(256) csr_vector_kernel(const int* __restrict__ rp, const int* __restrict__ col,
-                                                         const V* __restrict__ val, const float* __restrict__ x,
+                                                         const V* __restrict__ val, const float* x,
                                                          float* __restrict__ y, int m)
 {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(256) csr_vector_kernel(const int* __restrict__
     // rows past m keep their lanes in the shuffle with an empty segment
     const bool valid = row < m;
     const int s = valid ? __ldg(rp + row) : 0, e = valid ? __ldg(rp + row + 1) : 0;
+    grid_dependency();
     float acc = segment_dot<V, G>(col, val, x, s, e, lane);
     acc = group_sum<G>(acc);
     if (valid && lane == 0) y[row] += acc;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(256) csr_vector_kernel(const int* __restrict__
 // group per row).
 template <class V, int THREADS>
 __global__ void __launch_bounds__(THREADS) csr_block_row_kernel(const int* __restrict__ rp, const int* __restrict__ col,
-                                                                const V* __restrict__ val, const float* __restrict__ x,
+                                                                const V* __restrict__ val, const float* x,
                                                                 float* __restrict__ y, int m)
 {
     __shared__ float red[THREADS / 32];
@@ -301,7 +302,7 @@ constexpr int kCooChunk = 128 * kCooTiles;
 
 template <class V>
 __global__ void __launch_bounds__(256) coo_segment_kernel(const int* __restrict__ rowid, const int* __restrict__ colid,
-                                                          const V* __restrict__ val, const float* __restrict__ x,
+                                                          const V* __restrict__ val, const float* x,
                                                           float* __restrict__ y, int nnz_pad, int nwarps,
                                                           const int* __restrict__ span_of_head, const int4* __restrict__ spans,
                                                           int* __restrict__ span_count, float* __restrict__ part_val)
@@ -324,6 +325,7 @@ __global__ void __launch_bounds__(256) coo_segment_kernel(const int* __restrict_
     int4 rn = ld_int4(rowid + base + 4 * lane);
     int4 cn = ld_int4(colid + base + 4 * lane);
     float4 an = Val<V>::ld4(val + base + 4 * lane);
+    grid_dependency();
     for (int t = base; t < end; t += 128) {
         const int4 r = rn;
         const int4 c = cn;
@@ -339,8 +341,8 @@ __global__ void __launch_bounds__(256) coo_segment_kernel(const int* __restrict_
         // lane that closes it (head and tail rows go to the scratch pairs instead), so
         // the value read is still the original y.
         const float y0 = y[r.x], y1 = y[r.y], y2 = y[r.z], y3 = y[r.w];
-        const float p0 = a.x * ldx(x, c.x), p1 = a.y * ldx(x, c.y);
-        const float p2 = a.z * ldx(x, c.z), p3 = a.w * ldx(x, c.w);
+        const float p0 = a.x * x[c.x], p1 = a.y * x[c.y];
+        const float p2 = a.z * x[c.z], p3 = a.w * x[c.w];
         // the segment carried out of the previous tile ends if this tile starts a new row
         const int tile_first = __shfl_sync(0xffffffffu, r.x, 0);
         if (tile_first != carry_row) {

@@ -219,8 +219,7 @@ template <class V, int BH, int BW, int CW> struct SpmmShape {
 // K: the number of right-hand sides where it is known (0: `k_arg`).
 template <class V, int BH, int BW, int CW, int K>
 __global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V, BH, BW, CW>::ctas)
-    bcsr_spmm_stream_kernel(const int* __restrict__ rp, const unsigned* __restrict__ rec, const float* __restrict__ x,
-                            float* __restrict__ y, int nbr, int m, int k_arg, int rows)
+    bcsr_spmm_stream_kernel(const int* __restrict__ rp, const unsigned* __restrict__ rec, const float* x, float* y, int nbr, int m, int k_arg, int rows)
 {
     using Sh = SpmmShape<V, BH, BW, CW>;
     using Rec = BlockRec<V, BH * BW>;
@@ -260,10 +259,11 @@ __global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V
     for (int c0 = 0; c0 < k; c0 += 4 * CW) {
         const int c = c0 + 4 * cw;
         const bool writer = c < k;
-        const char* __restrict__ xc = reinterpret_cast<const char*>(x + (c < k ? c : 0));
-        float* __restrict__ yp = y + (size_t)r0 * BH * k + c + comp;   // this lane's Y entry of the row's first line
+        const char* xc = reinterpret_cast<const char*>(x + (c < k ? c : 0));
+        float* yp = y + (size_t)r0 * BH * k + c + comp;   // this lane's Y entry of the row's first line
         issue(0);
         issue(1);
+        if (c0 == 0) grid_dependency();
         int next = 0;               // chunks 0 .. next - 1 have landed
         int j = sb, r = r0, re = sb;
         float4 acc[BH];
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V
                 const unsigned off = t < re ? bk[u][Rec::xrow_word] : 0u;
                 const char* xp = xc + (size_t)off * 16;
 #pragma unroll
-                for (int w = 0; w < BW; w++) xv[u][w] = __ldg(reinterpret_cast<const float4*>(xp + w * kb));
+                for (int w = 0; w < BW; w++) xv[u][w] = *reinterpret_cast<const float4*>(xp + w * kb);
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {

@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpanel_kernel(const int* __rest
     float* xs = reinterpret_cast<float*>(xp_smem + xpanel_ring_bytes<V>());
     const int t_begin = (int)((long long)blockIdx.x * ntiles / gridDim.x);
     const int t_end = (int)((long long)(blockIdx.x + 1) * ntiles / gridDim.x);
+    grid_dependency();
     if (t_begin >= t_end) return;
     // panel holding t_begin: the last p with tile0[p] <= t_begin
     int lo = 0, hi = npanels - 1;
@@ -211,7 +212,9 @@ __global__ void __launch_bounds__(256) xpanel_merge_kernel(const int* __restrict
         const int a = __ldg(run_ptr + i), b = __ldg(run_ptr + i + 1);
         if (b - a > kXpShortRuns) return;
         const int r = run_rows ? __ldg(run_rows + i) : i;
+        // no other writer of a listed row's y in xpanel_kernel: only the partials are waited for
         const float yv = y[r];
+        grid_dependency();
         float q[kXpShortRuns];
 #pragma unroll
         for (int k = 0; k < kXpShortRuns; k++) q[k] = a + k < b ? partial[a + k] : 0.0f;
@@ -227,6 +230,7 @@ __global__ void __launch_bounds__(256) xpanel_merge_kernel(const int* __restrict
     // groups past the list keep their lanes in the shuffle with an empty range
     const int i = valid ? __ldg(long_list + g) : 0;
     const int a = valid ? __ldg(run_ptr + i) : 0, b = valid ? __ldg(run_ptr + i + 1) : 0;
+    grid_dependency();
     float s = 0.0f;
 #pragma unroll 4
     for (int j = a + lane; j < b; j += kXpMergeLanes) s += partial[j];
