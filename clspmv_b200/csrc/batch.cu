@@ -23,6 +23,7 @@
 #include "csp/clspmv.h"
 #include "internal.h"
 #include "engine.h"
+#include "launch.h"
 #include "kernels/batch.cuh"
 
 namespace csp {
@@ -34,7 +35,7 @@ namespace {
         if (_e != cudaSuccess) return cuda_error(_e, #call);        \
     } while (0)
 
-constexpr int kItemSlots = 2048;   // target stored slots per (warp) work item
+constexpr int kItemSlots = 1024;   // stored slots per (warp) work item, at most about
 
 inline long long pad_ll(long long v, long long a) { return (v + a - 1) / a * a; }
 
@@ -217,6 +218,7 @@ struct HPart {
     std::vector<int4> blocks, longs;
     int npartial = 0;
     long long slots = 0;            // stored slots (gradient length)
+    int item_slots = kItemSlots;    // slots per work item (cut_items)
     std::vector<dev::BatchItem> ranges;   // work items (part index filled in later)
 };
 
@@ -231,7 +233,7 @@ dev::BatchItem range_item(int v0, int v1, int4 blk = make_int4(0, 0, 0, 0))
     return it;
 }
 
-// groups consecutive virtual blocks into items of about kItemSlots slots
+// groups consecutive virtual blocks into items of about p.item_slots slots
 void cut_items(HPart& p, int nvb, const std::vector<long long>& vb_slots)
 {
     p.ranges.clear();
@@ -239,7 +241,7 @@ void cut_items(HPart& p, int nvb, const std::vector<long long>& vb_slots)
     long long acc = 0;
     for (int vb = 0; vb < nvb; vb++) {
         acc += vb_slots[vb];
-        if (acc >= kItemSlots || vb == nvb - 1) {
+        if (acc >= p.item_slots || vb == nvb - 1) {
             p.ranges.push_back(range_item(start, vb + 1));
             start = vb + 1;
             acc = 0;
@@ -272,13 +274,17 @@ void make_warp_blocks(const std::vector<int>& rp, int m, std::vector<int4>& bloc
         }
         const int start = r;
         long long acc = 0;
+        int longest = 0;
         while (r < m && r - start < dev::kWarpRows) {
             const int l = rp[r + 1] - rp[r];
             if (l > dev::kWarpNnz || acc + l > dev::kWarpNnz) break;
             acc += l;
+            longest = std::max(longest, l);
             r++;
         }
-        blocks.push_back(make_int4(start, r - start, rp[start], rp[r]));
+        const int nr = r - start;
+        blocks.push_back(make_int4(start, nr | (longest > dev::kAdaptSerial * dev::warp_row_lanes(nr) ? dev::kAdaptSkewed : 0),
+                                   rp[start], rp[r]));
     }
 }
 
@@ -519,16 +525,15 @@ int occupancy_grid(bool bf16, int nitems)
     return std::max(1, std::min(g, (nitems + dev::kBatchWarps - 1) / dev::kBatchWarps));
 }
 
-// One launch over `nitems` items: the item counter zeroed on the stream, then the kernel.
+// One launch over `nitems` items; `counter`: two ints, zero before the first launch.
 int launch_batch(bool bf16, const dev::BatchPart* parts, const dev::BatchItem* items, int nitems, int* counter,
                  unsigned long long* cycles, int grid, cudaStream_t st)
 {
     if (nitems <= 0) return CSP_OK;
-    BCUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
-    if (bf16)
-        dev::batch_kernel<__nv_bfloat16><<<grid, dev::kBatchThreads, 0, st>>>(parts, items, nitems, counter, cycles);
-    else
-        dev::batch_kernel<float><<<grid, dev::kBatchThreads, 0, st>>>(parts, items, nitems, counter, cycles);
+    // the last 16 items a warp are handed out one by one (8: 421 -> 452 us on 128 mixed matrices)
+    const int tail = 16 * grid * dev::kBatchWarps;
+    if (bf16) launch_chained(dev::batch_kernel<__nv_bfloat16>, grid, dev::kBatchThreads, 0, st, parts, items, nitems, tail, counter, cycles);
+    else launch_chained(dev::batch_kernel<float>, grid, dev::kBatchThreads, 0, st, parts, items, nitems, tail, counter, cycles);
     BCUDA(cudaGetLastError());
     return CSP_OK;
 }
@@ -613,23 +618,29 @@ struct csp_batch {
 
 namespace {
 
-// Builds the item list of one direction set from per-part ranges.
+// Builds the item list of one direction set from per-part ranges: the items that gather x
+// at random (CSR, SELL) first, then the streaming ones (DIA, BCSR), each in matrix order.  The
+// chip then runs one kind at a time out of its instruction cache and ends on short items
+// (128 mixed matrices, forward + adjoint, one B200: matrix order 407 us, the two kinds in
+// turn 398-411, gathers first 394).
 std::vector<dev::BatchItem> items_for(const csp_batch* b, int what)
 {
-    std::vector<dev::BatchItem> it;
+    std::vector<dev::BatchItem> gathers, streams;
     const int n = b->n;
-    auto add = [&](const std::vector<dev::BatchItem>& rs, int part) {
+    auto add = [&](const std::vector<dev::BatchItem>& rs, int part, int fmt) {
+        auto& to = fmt == CSP_BFMT_CSR || fmt == CSP_BFMT_SELL32 || fmt == CSP_BFMT_SELL128 ? gathers : streams;
         for (dev::BatchItem r : rs) {
             r.part = part;
-            it.push_back(r);
+            to.push_back(r);
         }
     };
     for (int i = 0; i < n; i++) {
-        if (what & CSP_BATCH_FWD) add(b->ranges_fwd[i], (what & CSP_BATCH_ADJ) ? n + i : i);
-        else if (what & CSP_BATCH_ADJ) add(b->ranges_fwd[i], 2 * n + i);
-        if (what & CSP_BATCH_ADJ) add(b->ranges_adj[i], 3 * n + i);
+        if (what & CSP_BATCH_FWD) add(b->ranges_fwd[i], (what & CSP_BATCH_ADJ) ? n + i : i, b->fmt[i]);
+        else if (what & CSP_BATCH_ADJ) add(b->ranges_fwd[i], 2 * n + i, b->fmt[i]);
+        if (what & CSP_BATCH_ADJ) add(b->ranges_adj[i], 3 * n + i, b->fmt_t[i]);
     }
-    return it;
+    gathers.insert(gathers.end(), streams.begin(), streams.end());
+    return gathers;
 }
 
 // Device timing of candidate formats for one side of the batch -- the stored matrices
@@ -699,7 +710,7 @@ int tune_classes(const std::vector<HCsr>& M, const std::vector<csp_batch_feature
             }
         const size_t o_items = ar.stage(items);
         const size_t o_cyc = ar.take(hp.size() * 8);
-        const size_t o_ctr = ar.take(sizeof(int));
+        const size_t o_ctr = ar.take(2 * sizeof(int));
         if ((rc = ar.commit())) break;
         std::vector<dev::BatchPart> d;
         for (int q = 0; q < (int)hp.size(); q++) {
@@ -718,7 +729,9 @@ int tune_classes(const std::vector<HCsr>& M, const std::vector<csp_batch_feature
         auto* ditems = reinterpret_cast<const dev::BatchItem*>(ar.base + o_items);
         auto* cyc = reinterpret_cast<unsigned long long*>(ar.base + o_cyc);
         auto* ctr = reinterpret_cast<int*>(ar.base + o_ctr);
-        rc = launch_batch(bf16, parts, ditems, (int)items.size(), ctr, nullptr, grid, st);
+        e = cudaMemsetAsync(ctr, 0, 2 * sizeof(int), st);
+        if (e != cudaSuccess) rc = cuda_error(e, "batch tuning");
+        if (!rc) rc = launch_batch(bf16, parts, ditems, (int)items.size(), ctr, nullptr, grid, st);
         if (!rc) {
             e = cudaMemsetAsync(cyc, 0, hp.size() * 8, st);
             if (e != cudaSuccess) rc = cuda_error(e, "batch tuning");
@@ -877,7 +890,13 @@ int csp_batch_create(const coo_matrix_if* const* mats, int n, const csp_batch_op
     b->ranges_fwd.resize((size_t)n);
     b->ranges_adj.resize((size_t)n);
     Arena& ar = b->arena;
+    // items small enough that a small batch has two for every warp of the chip (148 SMs x 32)
+    long long entries = 0;
+    for (int i = 0; i < n; i++) entries += F[i].nnz;
+    const int item_slots = (int)std::min<long long>(kItemSlots, std::max<long long>(1, entries * (b->adjoint ? 2 : 1) / (2 * 148 * 32)));
     for (int i = 0; i < n; i++) {
+        fw[i].item_slots = item_slots;
+        if (b->adjoint) bw[i].item_slots = item_slots;
         build_part(b->fmt[i], A[i], fw[i]);
         fo[i] = stage_part(ar, fw[i], b->bf16);
         b->ranges_fwd[i] = fw[i].ranges;
@@ -910,7 +929,7 @@ int csp_batch_create(const coo_matrix_if* const* mats, int n, const csp_batch_op
         o_ys = ar.take(ny * 4 + 16);
     }
     const size_t o_parts = ar.take((size_t)4 * n * sizeof(dev::BatchPart));
-    const size_t o_ctr = ar.take(sizeof(int));
+    const size_t o_ctr = ar.take(2 * sizeof(int));
     const int whats[3] = {CSP_BATCH_FWD, CSP_BATCH_ADJ, CSP_BATCH_FWD | CSP_BATCH_ADJ};
     size_t o_items[4] = {0, 0, 0, 0};
     for (int w : whats) {
@@ -951,6 +970,7 @@ int csp_batch_create(const coo_matrix_if* const* mats, int n, const csp_batch_op
     }
     b->dparts = reinterpret_cast<dev::BatchPart*>(base + o_parts);
     BCUDA(cudaMemcpy(b->dparts, b->hparts.data(), b->hparts.size() * sizeof(dev::BatchPart), cudaMemcpyHostToDevice));
+    BCUDA(cudaMemset(b->counter, 0, 2 * sizeof(int)));
     for (int w : whats) {
         b->ditems[w] = reinterpret_cast<dev::BatchItem*>(base + o_items[w]);
         b->grid[w] = occupancy_grid(b->bf16, std::max(1, b->nitems[w]));
