@@ -21,11 +21,12 @@
 #include "csp/clspmv.h"
 #include "internal.h"
 #include "engine.h"
+#include "launch.h"
 #include "kernels/common.cuh"
 
 namespace csp {
 
-constexpr int kNoAllocChunk = 512;                                        // entries per warp
+constexpr int kNoAllocChunk = 512;                                        // entries per warp, at most
 constexpr int kNoAllocMaxWarps = CSP_NOALLOC_MAX_NNZ / kNoAllocChunk;     // 65,536
 static_assert(CSP_NOALLOC_SCRATCH_BYTES == 2 * kNoAllocMaxWarps * (4 + 4), "scratch holds 2 (row, sum) pairs per warp");
 
@@ -35,14 +36,13 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[CSP_NOALLOC_SCR
 
 namespace {
 
-__device__ __forceinline__ void load_entry(const int* __restrict__ rowid, const int* __restrict__ colid,
-                                           const float* __restrict__ val, int j, int nnz, int last_row,
+__device__ __forceinline__ void load_entry(const int* rowid, const int* colid, const float* val, int j, int nnz, int last_row,
                                            int& r, int& c, float& v)
 {
     if (j < nnz) {
-        r = __ldg(rowid + j);
-        c = __ldg(colid + j);
-        v = __ldg(val + j);
+        r = rowid[j];
+        c = colid[j];
+        v = val[j];
     } else {   // padding past the caller's arrays: extends the last row by zeros
         r = last_row;
         c = 0;
@@ -50,9 +50,9 @@ __device__ __forceinline__ void load_entry(const int* __restrict__ rowid, const 
     }
 }
 
-__device__ __forceinline__ float x_at(const float* __restrict__ x, int c, int width)
+__device__ __forceinline__ float x_at(const float* x, int c, int width)
 {
-    return (c >= 0 && c < width) ? __ldg(x + c) : 0.0f;
+    return (c >= 0 && c < width) ? x[c] : 0.0f;
 }
 
 __device__ __forceinline__ float y_at(const float* y, int r, int height)
@@ -60,40 +60,65 @@ __device__ __forceinline__ float y_at(const float* y, int r, int height)
     return (r >= 0 && r < height) ? y[r] : 0.0f;
 }
 
-__global__ void __launch_bounds__(256) coo_noalloc_segment(const int* __restrict__ rowid, const int* __restrict__ colid,
-                                                           const float* __restrict__ val, const float* __restrict__ x,
-                                                           float* __restrict__ y, int nnz, int height, int width, int nwarps,
+// One tile of 128 entries, four consecutive ones per lane.
+struct Tile {
+    int4 r, c;
+    float4 a;
+};
+
+// Each warp reduces `chunk` entries (two or four tiles), tile by tile.  Latency is what bounds it (a few
+// thousand warps, three dependent steps a tile), so the steps overlap: while tile t is
+// reduced, the gathers of x and y for tile t + 1 and the entries of tile t + 2 are in
+// flight.  Past that the L1's gather rate (a line a clock) is the limit.  300,007 Zipf rows,
+// 1.9 M entries, one B200: 31 us a call (segment 16, fix-up 8, and the launches) -> 24.  A row closed inside the chunk is written by the lane that closes it; the
+// chunk's first and last row go to the scratch pairs.
+__global__ void __launch_bounds__(256) coo_noalloc_segment(const int* rowid, const int* colid, const float* val, const float* x,
+                                                           float* y, int nnz, int height, int width, int nwarps, int chunk,
                                                            int* __restrict__ part_row, float* __restrict__ part_val)
 {
+    dev::grid_dependency();   // the caller's arrays may be written by the operation before
     const int lane = threadIdx.x & 31;
     const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (w >= nwarps) return;
-    const int last_row = __ldg(rowid + nnz - 1);
+    const int last_row = rowid[nnz - 1];
     const int nnz_tiles = (nnz + 127) / 128 * 128;
-    const int base = w * kNoAllocChunk;
-    const int end = min(base + kNoAllocChunk, nnz_tiles);
-    const int head_row = __ldg(rowid + base);
+    const int base = w * chunk;
+    const int end = min(base + chunk, nnz_tiles);
+    const int head_row = rowid[base];
     bool head_open = true;
     int carry_row = head_row;
-    float carry_val = 0.0f;
-    for (int t = base; t < end; t += 128) {
+    float carry_val = 0.0f, carry_y = 0.0f;
+    auto load = [&](int t, Tile& q) {
         const int j = t + 4 * lane;
-        int4 r;
-        int4 c;
-        float4 a;
         if (t + 128 <= nnz) {
-            r = dev::ld_int4(rowid + j);
-            c = dev::ld_int4(colid + j);
-            a = dev::Val<float>::ld4(val + j);
+            q.r = *reinterpret_cast<const int4*>(rowid + j);
+            q.c = *reinterpret_cast<const int4*>(colid + j);
+            q.a = *reinterpret_cast<const float4*>(val + j);
         } else {
-            load_entry(rowid, colid, val, j + 0, nnz, last_row, r.x, c.x, a.x);
-            load_entry(rowid, colid, val, j + 1, nnz, last_row, r.y, c.y, a.y);
-            load_entry(rowid, colid, val, j + 2, nnz, last_row, r.z, c.z, a.z);
-            load_entry(rowid, colid, val, j + 3, nnz, last_row, r.w, c.w, a.w);
+            load_entry(rowid, colid, val, j + 0, nnz, last_row, q.r.x, q.c.x, q.a.x);
+            load_entry(rowid, colid, val, j + 1, nnz, last_row, q.r.y, q.c.y, q.a.y);
+            load_entry(rowid, colid, val, j + 2, nnz, last_row, q.r.z, q.c.z, q.a.z);
+            load_entry(rowid, colid, val, j + 3, nnz, last_row, q.r.w, q.c.w, q.a.w);
         }
-        const float y0 = y_at(y, r.x, height), y1 = y_at(y, r.y, height), y2 = y_at(y, r.z, height), y3 = y_at(y, r.w, height);
-        const float p0 = a.x * x_at(x, c.x, width), p1 = a.y * x_at(x, c.y, width);
-        const float p2 = a.z * x_at(x, c.z, width), p3 = a.w * x_at(x, c.w, width);
+    };
+    auto gather = [&](const Tile& q, float4& xv, float4& yv) {
+        xv = make_float4(x_at(x, q.c.x, width), x_at(x, q.c.y, width), x_at(x, q.c.z, width), x_at(x, q.c.w, width));
+        yv = make_float4(y_at(y, q.r.x, height), y_at(y, q.r.y, height), y_at(y, q.r.z, height), y_at(y, q.r.w, height));
+    };
+    Tile cur, nxt;
+    float4 xv, yv;
+    load(base, cur);
+    if (base + 128 < end) load(base + 128, nxt);
+    gather(cur, xv, yv);
+    for (int t = base; t < end; t += 128) {
+        const int4 r = cur.r;
+        const float p0 = cur.a.x * xv.x, p1 = cur.a.y * xv.y, p2 = cur.a.z * xv.z, p3 = cur.a.w * xv.w;
+        const float4 y4 = yv;
+        if (t + 128 < end) {
+            cur = nxt;
+            if (t + 256 < end) load(t + 256, nxt);
+            gather(cur, xv, yv);
+        }
         const int tile_first = __shfl_sync(0xffffffffu, r.x, 0);
         if (tile_first != carry_row) {
             if (lane == 0) {
@@ -101,7 +126,7 @@ __global__ void __launch_bounds__(256) coo_noalloc_segment(const int* __restrict
                     part_row[2 * w] = carry_row;
                     part_val[2 * w] = carry_val;
                 } else if (carry_row >= 0 && carry_row < height) {
-                    y[carry_row] += carry_val;
+                    y[carry_row] = carry_y + carry_val;
                 }
             }
             if (head_open && carry_row == head_row) head_open = false;
@@ -125,12 +150,12 @@ __global__ void __launch_bounds__(256) coo_noalloc_segment(const int* __restrict
         bool closed_head = false;
         const int rr[4] = {r.x, r.y, r.z, r.w};
         const float pp[4] = {p0, p1, p2, p3};
-        const float yy[4] = {y0, y1, y2, y3};
+        const float yy[4] = {y4.x, y4.y, y4.z, y4.w};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             run += pp[k];
-            const int nxt = (k == 3) ? next_first : rr[k + 1];
-            const bool closes = (k < 3) ? (nxt != rr[k]) : (lane < 31 && nxt != rr[k]);
+            const int nx = (k == 3) ? next_first : rr[k + 1];
+            const bool closes = (k < 3) ? (nx != rr[k]) : (lane < 31 && nx != rr[k]);
             if (closes) {
                 if (head_open && rr[k] == head_row) {
                     part_row[2 * w] = rr[k];
@@ -144,6 +169,7 @@ __global__ void __launch_bounds__(256) coo_noalloc_segment(const int* __restrict
         }
         carry_row = __shfl_sync(0xffffffffu, r.w, 31);
         carry_val = __shfl_sync(0xffffffffu, run, 31);
+        carry_y = __shfl_sync(0xffffffffu, y4.w, 31);
         if (__any_sync(0xffffffffu, closed_head)) head_open = false;
     }
     if (lane == 0) {
@@ -159,16 +185,58 @@ __global__ void __launch_bounds__(256) coo_noalloc_segment(const int* __restrict
     }
 }
 
+// Adds each row's consecutive scratch pairs to y.  A warp takes 32 pairs: a keyed scan over
+// the lanes sums the runs that start in it, and the run that reaches its last lane is
+// followed through the next pairs 32 at a time (a row of 10,000 entries has 40 pairs: one
+// thread per run read them one after the other, 8 us of a 300,007-row Zipf product).  Runs
+// that start in an earlier warp's pairs are that warp's.
 __global__ void __launch_bounds__(256) coo_noalloc_fixup(const int* __restrict__ part_row, const float* __restrict__ part_val,
-                                                         int nparts, int height, float* __restrict__ y)
+                                                         int nparts, int height, float* y)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nparts) return;
-    const int r = part_row[i];
-    if (i > 0 && part_row[i - 1] == r) return;
-    float acc = 0.0f;
-    for (int k = i; k < nparts && part_row[k] == r; k++) acc += part_val[k];
-    if (r >= 0 && r < height) y[r] += acc;
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    const int lane = threadIdx.x & 31, first = i - lane;
+    dev::grid_dependency();
+    if (first >= nparts) return;   // the whole warp leaves together
+    // plain loads: the pairs are written within the life of this waiting kernel
+    const volatile int* prow = part_row;
+    const volatile float* pval = part_val;
+    const bool valid = i < nparts;
+    const int r = valid ? prow[i] : 0;
+    const float v = valid ? pval[i] : 0.0f;
+    const float y0 = valid ? y_at(y, r, height) : 0.0f;
+    const int before = lane == 0 && i > 0 ? prow[i - 1] : 0;
+    const int up = __shfl_up_sync(0xffffffffu, r, 1);
+    const bool head = valid && (i == 0 || (lane == 0 ? before : up) != r);
+    const unsigned heads = __ballot_sync(0xffffffffu, head), valids = __ballot_sync(0xffffffffu, valid);
+    if (!heads) return;
+    // this lane's run starts at lane `start` (none: it starts in an earlier warp)
+    const unsigned below = heads & (0xffffffffu >> (31 - lane));
+    const int start = below ? 31 - __clz(below) : -1;
+    float sum = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const float o = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane - d >= max(start, 0)) sum += o;
+    }
+    const bool last = valid && (lane == 31 || ((heads >> (lane + 1)) & 1u) || !((valids >> (lane + 1)) & 1u));
+    if ((valids >> 31) & 1u) {
+        // the run of lane 31 may go on
+        const int row = __shfl_sync(0xffffffffu, r, 31);
+        float more = 0.0f;
+        for (int j0 = first + 32; j0 < nparts; j0 += 32) {
+            const int j = j0 + lane;
+            const bool same = j < nparts && prow[j] == row;
+            const unsigned mism = __ballot_sync(0xffffffffu, !same);
+            const int n = mism ? __ffs(mism) - 1 : 32;
+            float t = lane < n ? pval[j] : 0.0f;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            more += t;
+            if (mism) break;
+        }
+        if (lane == 31) sum += more;
+    }
+    if (last && start >= 0 && r >= 0 && r < height) y[r] = y0 + sum;
 }
 
 // Device address of g_noalloc_scratch, looked up once per device with that device
@@ -221,11 +289,14 @@ extern "C" int csp_coo_spmv_noalloc(int height, int width, int nnz, const int* d
     if (rc) return rc;
     int* part_row = static_cast<int*>(scratch);
     float* part_val = reinterpret_cast<float*>(static_cast<char*>(scratch) + CSP_NOALLOC_SCRATCH_BYTES / 2);
-    const int nwarps = (nnz + kNoAllocChunk - 1) / kNoAllocChunk;
+    // two tiles a warp where that fills the chip's 148 x 32 warps at most once (100,000 Zipf rows:
+    // 13.4 us a call against 15.0 with four), four beyond (1 M rows: 47.3 against 48.0)
+    const int chunk = nnz <= 148 * 32 * kNoAllocChunk / 2 ? kNoAllocChunk / 2 : kNoAllocChunk;
+    const int nwarps = (nnz + chunk - 1) / chunk;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    coo_noalloc_segment<<<(nwarps * 32 + 255) / 256, 256, 0, st>>>(d_row, d_col, d_val, d_x, d_y, nnz, height, width, nwarps,
-                                                                   part_row, part_val);
-    coo_noalloc_fixup<<<(2 * nwarps + 255) / 256, 256, 0, st>>>(part_row, part_val, 2 * nwarps, height, d_y);
+    launch_chained(coo_noalloc_segment, (nwarps * 32 + 255) / 256, 256, 0, st, d_row, d_col, d_val, d_x, d_y, nnz, height, width,
+                   nwarps, chunk, part_row, part_val);
+    launch_chained(coo_noalloc_fixup, (2 * nwarps + 255) / 256, 256, 0, st, part_row, part_val, 2 * nwarps, height, d_y);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CSP_OK : cuda_error(e, "coo_spmv_noalloc launch");
 }
