@@ -36,11 +36,15 @@
 namespace csp {
 namespace dev {
 
-constexpr int kXpThreads = 512;
+// 32 warps of two stages each: as many bytes in flight as 16 of four, and twice the warps to
+// hide the shared-memory and shuffle latency of a tile (one B200, in a graph, kernel + merge:
+// 1 M Zipf rows 30.2 -> 29.2 us, 300,007 rows 14.0 -> 13.5, 60,000 rows 12.5 -> 11.4; 768 x 3
+// 30.7, 1024 x 3 30.5, which leaves less room for the panel)
+constexpr int kXpThreads = 1024;
 constexpr int kXpWarps = kXpThreads / 32;
 constexpr int kXpTile = 128;                // entries per tile: 4 per lane
 constexpr int kXpPanelMax = 65536;          // panel-local columns are 16-bit
-constexpr int kXpStages = 4;                // tiles in flight per warp
+constexpr int kXpStages = 2;                // tiles in flight per warp
 constexpr int kXpShortRuns = 8;             // rows with at most this many slots: a thread each
 constexpr int kXpMergeLanes = 8;            // lanes per longer row in the merge
 
@@ -109,7 +113,7 @@ template <class V>
 __global__ void __launch_bounds__(kXpThreads, 1) xpanel_kernel(const int* __restrict__ tile0, int ntiles, int npanels,
                                                                const int* __restrict__ slot,
                                                                const unsigned short* __restrict__ lcol,
-                                                               const V* __restrict__ val, const float* __restrict__ x,
+                                                               const V* __restrict__ val, const float* x,
                                                                int n, int panel_w, float* __restrict__ partial,
                                                                float* __restrict__ y)
 {
@@ -119,8 +123,10 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpanel_kernel(const int* __rest
     float* xs = reinterpret_cast<float*>(xp_smem + xpanel_ring_bytes<V>());
     const int t_begin = (int)((long long)blockIdx.x * ntiles / gridDim.x);
     const int t_end = (int)((long long)(blockIdx.x + 1) * ntiles / gridDim.x);
-    grid_dependency();
-    if (t_begin >= t_end) return;
+    if (t_begin >= t_end) {
+        grid_dependency();
+        return;
+    }
     // panel holding t_begin: the last p with tile0[p] <= t_begin
     int lo = 0, hi = npanels - 1;
     while (lo < hi) {
@@ -129,20 +135,25 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpanel_kernel(const int* __rest
     }
     int p = lo;
     int t = t_begin;
+    bool x_ready = false;
     while (t < t_end) {
         const int seg_end = min(t_end, __ldg(tile0 + p + 1));
         if (seg_end > t) {
-            // --- this panel of x into shared memory (x is zero-padded past n to a multiple of 64) ---
-            const int c0 = p * panel_w;
-            const int nv4 = (min(panel_w, n - c0) + 3) >> 2;
-            const float4* __restrict__ xg = reinterpret_cast<const float4*>(x + c0);
-            for (int i = threadIdx.x; i < nv4; i += kXpThreads) cp_async16(reinterpret_cast<float4*>(xs) + i, xg + i);
-            cp_async_commit();
-            // the first kXpStages - 1 tiles of this warp
+            // the first kXpStages - 1 tiles of this warp (constant: requested before x is waited for)
             const int first = t + warp;
 #pragma unroll
             for (int q = 0; q < kXpStages - 1; q++) xpanel_issue<V>(ring[q], first + q * kXpWarps, seg_end, lane, slot, lcol, val);
-            cp_async_wait<kXpStages - 1>();   // the x group (the oldest) has landed
+            if (!x_ready) {
+                grid_dependency();
+                x_ready = true;
+            }
+            // --- this panel of x into shared memory (x is zero-padded past n to a multiple of 64) ---
+            const int c0 = p * panel_w;
+            const int nv4 = (min(panel_w, n - c0) + 3) >> 2;
+            const float4* xg = reinterpret_cast<const float4*>(x + c0);
+            for (int i = threadIdx.x; i < nv4; i += kXpThreads) cp_async16(reinterpret_cast<float4*>(xs) + i, xg + i);
+            cp_async_commit();
+            cp_async_wait<0>();
             __syncthreads();
             int stage = 0;
             for (int tt = first; tt < seg_end; tt += kXpWarps) {
