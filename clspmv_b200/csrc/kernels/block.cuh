@@ -161,6 +161,12 @@ constexpr int kGbThreads = 128;   // 8 CTAs per SM at 64 registers: their load a
 constexpr int kGbBlocks = 4 * kGbThreads;
 constexpr int kGbRows = 128;
 
+// A CTA requests for L2 the blocks of the item half a wave of CTAs later (148 SMs x 8 CTAs), so
+// DRAM keeps working while the CTAs gather and reduce.  10 M 3x3 blocks, one B200, in a graph:
+// FP32 93.4 -> 86.3 us, BF16 80.9 -> 77.8; a quarter wave ahead 87.9, an eighth 92.7, one and a
+// half waves 89.9, two 94.5.
+constexpr unsigned kGbAhead = 148 * 4;
+
 // Row sums of one item: a lane group of G lanes per block row adds the row's block
 // products (prod, row order) and writes y = s_y + sum (s_y: the item's y rows).
 template <int BH, int G>
@@ -211,6 +217,14 @@ __global__ void __launch_bounds__(kGbThreads) bcsr_adaptive_kernel(const int* __
         tg = __ldg(reinterpret_cast<const uint2*>(tgt + j));
 #pragma unroll
         for (int k = 0; k < BH * BW; k++) d[k] = Val<V>::ld4(data + (size_t)k * aligned + j);
+    }
+    // the blocks of the item kGbAhead CTAs on go to L2, a plane per lane of the last warp
+    if (tid >= kGbThreads - 32 && blockIdx.x + kGbAhead < gridDim.x) {
+        const int4 nw = __ldg(work + blockIdx.x + kGbAhead);
+        const int l = tid - (kGbThreads - 32), slots = ((nw.y >> 16) + 3) & ~3;
+        if (l < BH * BW) prefetch_l2(data + (size_t)l * aligned + nw.w, slots * (int)sizeof(V));
+        else if (l == BH * BW) prefetch_l2(col + nw.w, slots * 4);
+        else if (l == BH * BW + 1) prefetch_l2(tgt + nw.w, slots * 2);
     }
     // the item's row pointers and y rows, requested with the blocks so that the y update
     // does not wait on DRAM

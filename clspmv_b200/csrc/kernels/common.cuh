@@ -62,6 +62,15 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src)
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// Requests the whole 16-byte units of [p, p + bytes) for L2, by one instruction; no result is
+// waited for.
+__device__ __forceinline__ void prefetch_l2(const void* p, int bytes)
+{
+    const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
+    const int n = (int)((reinterpret_cast<uintptr_t>(p) + bytes - a) & ~(uintptr_t)15);
+    if (n > 0 && bytes > 0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(a), "r"(n));
+}
+
 __device__ __forceinline__ int4 ld_int4(const int* p) { return __ldg(reinterpret_cast<const int4*>(p)); }
 __device__ __forceinline__ float ldx(const float* x, int i) { return __ldg(x + i); }
 __device__ __forceinline__ float4 ldx4(const float* x, int i) { return __ldg(reinterpret_cast<const float4*>(x + i)); }
