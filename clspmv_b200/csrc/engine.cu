@@ -708,8 +708,9 @@ int Engine::add_generic_bcsr(const bcsr_matrix_if& b, int method)
         fits = fits && !work.empty();
     }
     const int nblk = b.bcsr_block_num;
-    if (nrhs % 4 == 0 && !(tensor_spmm && nrhs % 32 == 0 && bw * bh <= 16)) {
-        // several right-hand sides in whole float4s: block records (kernels/spmm.cuh)
+    if (nrhs % 4 == 0 && !(tensor_spmm && nrhs % 32 == 0 && bw * bh <= 16) && (long long)width * (nrhs / 4) <= UINT32_MAX) {
+        // several right-hand sides in whole float4s, X rows indexed in 32 bits: block records
+        // (kernels/spmm.cuh)
         if ((rc = upload_block_records(p, b))) return rc;
     } else if (!fits) {
         if ((rc = upload_int(&p.i1, b.bcsr_col_id, nblk, (size_t)pad_to(nblk, 4) + 4)) ||

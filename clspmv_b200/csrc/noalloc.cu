@@ -12,7 +12,7 @@
 // until the process exits.  It bounds the matrix to CSP_NOALLOC_MAX_NNZ entries.
 //
 // The kernels restate the COO segmented reduction of kernels/flat.cuh
-// (coo_segment_kernel + coo_fixup_kernel) for unpadded caller arrays: the last tile
+// (coo_segment_kernel) for unpadded caller arrays, with a fix-up pass: the last tile
 // is read with masked scalar loads, and every row/column index is range-checked so a
 // malformed matrix gives a wrong result instead of an out-of-bounds access.
 #include <cuda_runtime.h>
