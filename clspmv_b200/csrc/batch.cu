@@ -525,15 +525,22 @@ int occupancy_grid(bool bf16, int nitems)
     return std::max(1, std::min(g, (nitems + dev::kBatchWarps - 1) / dev::kBatchWarps));
 }
 
+// How many of a list's leading items are handed out four at a time: the small ones that
+// gather x (252 entries at most), where single items would contend for the counter (a batch
+// of 43 Zipf matrices forward, 126 us against 117), up to the last eight a warp, where a warp
+// that holds several would finish after the others (two or four a warp: 119).
+int leading_fours(int gathers, int streams, int grid)
+{
+    return std::max(0, gathers - std::max(0, 8 * grid * dev::kBatchWarps - streams));
+}
+
 // One launch over `nitems` items; `counter`: two ints, zero before the first launch.
-int launch_batch(bool bf16, const dev::BatchPart* parts, const dev::BatchItem* items, int nitems, int* counter,
+int launch_batch(bool bf16, const dev::BatchPart* parts, const dev::BatchItem* items, int nitems, int fours, int* counter,
                  unsigned long long* cycles, int grid, cudaStream_t st)
 {
     if (nitems <= 0) return CSP_OK;
-    // the last 16 items a warp are handed out one by one (8: 421 -> 452 us on 128 mixed matrices)
-    const int tail = 16 * grid * dev::kBatchWarps;
-    if (bf16) launch_chained(dev::batch_kernel<__nv_bfloat16>, grid, dev::kBatchThreads, 0, st, parts, items, nitems, tail, counter, cycles);
-    else launch_chained(dev::batch_kernel<float>, grid, dev::kBatchThreads, 0, st, parts, items, nitems, tail, counter, cycles);
+    if (bf16) launch_chained(dev::batch_kernel<__nv_bfloat16>, grid, dev::kBatchThreads, 0, st, parts, items, nitems, fours, counter, cycles);
+    else launch_chained(dev::batch_kernel<float>, grid, dev::kBatchThreads, 0, st, parts, items, nitems, fours, counter, cycles);
     BCUDA(cudaGetLastError());
     return CSP_OK;
 }
@@ -599,7 +606,7 @@ struct csp_batch {
     std::vector<dev::BatchPart> hparts;      // [fwd(n) | fwd+grad(n) | grad only(n) | adj(n)]
     dev::BatchPart* dparts = nullptr;
     dev::BatchItem* ditems[4] = {nullptr, nullptr, nullptr, nullptr};   // by `what`
-    int nitems[4] = {0, 0, 0, 0};
+    int nitems[4] = {0, 0, 0, 0}, ngathers[4] = {0, 0, 0, 0}, fours[4] = {0, 0, 0, 0};
     int grid[4] = {1, 1, 1, 1};
     std::vector<std::vector<dev::BatchItem>> ranges_fwd, ranges_adj;   // per matrix
     std::vector<int> plain_g;                                 // csp_batch_run_plain lanes per row (A, A^T)
@@ -623,7 +630,7 @@ namespace {
 // chip then runs one kind at a time out of its instruction cache and ends on short items
 // (128 mixed matrices, forward + adjoint, one B200: matrix order 407 us, the two kinds in
 // turn 398-411, gathers first 394).
-std::vector<dev::BatchItem> items_for(const csp_batch* b, int what)
+std::vector<dev::BatchItem> items_for(const csp_batch* b, int what, int* ngathers)
 {
     std::vector<dev::BatchItem> gathers, streams;
     const int n = b->n;
@@ -639,6 +646,7 @@ std::vector<dev::BatchItem> items_for(const csp_batch* b, int what)
         else if (what & CSP_BATCH_ADJ) add(b->ranges_fwd[i], 2 * n + i, b->fmt[i]);
         if (what & CSP_BATCH_ADJ) add(b->ranges_adj[i], 3 * n + i, b->fmt_t[i]);
     }
+    *ngathers = (int)gathers.size();
     gathers.insert(gathers.end(), streams.begin(), streams.end());
     return gathers;
 }
@@ -725,19 +733,21 @@ int tune_classes(const std::vector<HCsr>& M, const std::vector<csp_batch_feature
         cudaError_t e = cudaMemcpy(ar.base + o_parts, d.data(), d.size() * sizeof(dev::BatchPart), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) { rc = cuda_error(e, "batch tuning upload"); ar.release(); break; }
         const int grid = occupancy_grid(bf16, (int)items.size());
+        const bool gathers = fmt == CSP_BFMT_CSR || fmt == CSP_BFMT_SELL32 || fmt == CSP_BFMT_SELL128;
+        const int fours = gathers ? leading_fours((int)items.size(), 0, grid) : 0;
         auto* parts = reinterpret_cast<const dev::BatchPart*>(ar.base + o_parts);
         auto* ditems = reinterpret_cast<const dev::BatchItem*>(ar.base + o_items);
         auto* cyc = reinterpret_cast<unsigned long long*>(ar.base + o_cyc);
         auto* ctr = reinterpret_cast<int*>(ar.base + o_ctr);
         e = cudaMemsetAsync(ctr, 0, 2 * sizeof(int), st);
         if (e != cudaSuccess) rc = cuda_error(e, "batch tuning");
-        if (!rc) rc = launch_batch(bf16, parts, ditems, (int)items.size(), ctr, nullptr, grid, st);
+        if (!rc) rc = launch_batch(bf16, parts, ditems, (int)items.size(), fours, ctr, nullptr, grid, st);
         if (!rc) {
             e = cudaMemsetAsync(cyc, 0, hp.size() * 8, st);
             if (e != cudaSuccess) rc = cuda_error(e, "batch tuning");
         }
         const int reps = 3;
-        for (int k = 0; k < reps && !rc; k++) rc = launch_batch(bf16, parts, ditems, (int)items.size(), ctr, cyc, grid, st);
+        for (int k = 0; k < reps && !rc; k++) rc = launch_batch(bf16, parts, ditems, (int)items.size(), fours, ctr, cyc, grid, st);
         std::vector<unsigned long long> hc(hp.size());
         if (!rc) {
             e = cudaMemcpyAsync(hc.data(), cyc, hp.size() * 8, cudaMemcpyDeviceToHost, st);
@@ -934,7 +944,7 @@ int csp_batch_create(const coo_matrix_if* const* mats, int n, const csp_batch_op
     size_t o_items[4] = {0, 0, 0, 0};
     for (int w : whats) {
         if ((w & CSP_BATCH_ADJ) && !b->adjoint) continue;
-        std::vector<dev::BatchItem> it = items_for(b.get(), w);
+        std::vector<dev::BatchItem> it = items_for(b.get(), w, &b->ngathers[w]);
         b->nitems[w] = (int)it.size();
         o_items[w] = ar.stage(it);
     }
@@ -974,6 +984,7 @@ int csp_batch_create(const coo_matrix_if* const* mats, int n, const csp_batch_op
     for (int w : whats) {
         b->ditems[w] = reinterpret_cast<dev::BatchItem*>(base + o_items[w]);
         b->grid[w] = occupancy_grid(b->bf16, std::max(1, b->nitems[w]));
+        b->fours[w] = leading_fours(b->ngathers[w], b->nitems[w] - b->ngathers[w], b->grid[w]);
     }
     *out = b.release();
     return CSP_OK;
@@ -1056,7 +1067,7 @@ int csp_batch_run(csp_batch* b, int what, int ntimes)
     cudaStream_t st = b->stream;
     if (!b->use_graph) {
         for (int k = 0; k < ntimes; k++) {
-            int rc = launch_batch(b->bf16, b->dparts, b->ditems[what], b->nitems[what], b->counter, nullptr, b->grid[what], st);
+            int rc = launch_batch(b->bf16, b->dparts, b->ditems[what], b->nitems[what], b->fours[what], b->counter, nullptr, b->grid[what], st);
             if (rc) return rc;
         }
         return CSP_OK;
@@ -1065,7 +1076,7 @@ int csp_batch_run(csp_batch* b, int what, int ntimes)
         if (b->graph[what]) { cudaGraphExecDestroy(b->graph[what]); b->graph[what] = nullptr; }
         cudaGraph_t g;
         BCUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        int rc = launch_batch(b->bf16, b->dparts, b->ditems[what], b->nitems[what], b->counter, nullptr, b->grid[what], st);
+        int rc = launch_batch(b->bf16, b->dparts, b->ditems[what], b->nitems[what], b->fours[what], b->counter, nullptr, b->grid[what], st);
         cudaError_t e = cudaStreamEndCapture(st, &g);
         if (rc) { if (e == cudaSuccess) cudaGraphDestroy(g); return rc; }
         if (e != cudaSuccess) return cuda_error(e, "cudaStreamEndCapture");

@@ -42,7 +42,7 @@ constexpr int kBatchDiaRows = 4 * 32;            // DIA step: four consecutive r
 constexpr int kBatchSellRows = 32;               // SELL step: a row per lane
 constexpr int kBatchBcsrLanes = 2;               // BCSR: lanes per block row
 constexpr int kBatchBcsrRows = 32 / kBatchBcsrLanes;   // BCSR step: block rows per warp
-constexpr int kBatchTake = 4;                    // items a warp takes from the counter at once, far from the list's end
+constexpr int kBatchTake = 4;                    // small items a warp takes from the counter at once
 
 struct BatchPart {
     int kind;
@@ -459,8 +459,7 @@ __device__ __forceinline__ void cp_async_commit_wait_all() { asm volatile("cp.as
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::); }
 
 // Warp w starts with item w; further items come from a shared counter, kBatchTake
-// consecutive ones per atomic -- one within the last `tail` items, where a warp that holds
-// several would finish after the others.  A warp takes the item after its next one while it
+// consecutive ones per atomic among the first `fours` items, one after them.  A warp takes the item after its next one while it
 // runs the current item, so the items a warp gets follow how long its earlier ones took.
 // The next item's descriptor and the words of the item after it are copied into the warp's
 // shared memory asynchronously (cp.async) while the current item runs, so no register holds
@@ -470,7 +469,7 @@ __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async
 // held a warp (the autotuner's cost).
 template <class V>
 __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPart* __restrict__ parts,
-                                                                  const BatchItem* __restrict__ items, int nitems, int tail,
+                                                                  const BatchItem* __restrict__ items, int nitems, int fours,
                                                                   int* __restrict__ next,
                                                                   unsigned long long* __restrict__ cycles)
 {
@@ -484,7 +483,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPart
         int v = 0;
         if (lane == 0) {
             if (ws.res_next == ws.res_end) {
-                const int take = ws.res_end < nitems - tail ? kBatchTake : 1;
+                const int take = ws.res_end < fours ? kBatchTake : 1;
                 ws.res_next = nwarps + atomicAdd(next, take);
                 ws.res_end = ws.res_next + take;
             }

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(THREADS) csr_block_row_kernel(const int* __res
 // block's row count and written once (y = y + sum).  Where a row is much longer than its
 // block's mean (the host flags the block) one lane would add up to 2040 products one after
 // the other; such rows are listed and summed by a warp each.  On 200,003 Zipf rows (1.3 M
-// entries, one B200, in a graph) the kernel takes 12.4 us instead of 16.4, on 50,003 rows 5.9
+// entries, one B200, in a graph) the kernel takes 11.9 us instead of 16.6, on 50,000 rows 5.2
 // instead of 9.0; work blocks of up to 1024 rows instead of 256 are 1 us faster there and
 // 1 us slower on 1 M and on 50,003 rows.  A chunk of a long row writes
 // its partial sum to a scratch slot; the CTA that finishes a row's last chunk (an
@@ -149,7 +149,9 @@ constexpr int kAdaptVecs = (kAdaptNnz + 3) / 4 + 1;  // 511
 constexpr int kAdaptSkewed = 1 << 16;                // row-count flag: a block with rows longer than its lane groups take
 
 // A row with more entries than this per lane of its group is left to a whole warp.
-constexpr int kAdaptSerial = 16;
+// (16 makes a warp of 30- to 90-entry rows, a FEM matrix as CSR, slower than lane groups: 19.0 us
+// instead of 17.0 at 40,000 block rows; 64 is as fast as 32.)
+constexpr int kAdaptSerial = 32;
 
 // Lanes per row for a block of nrows rows.
 __host__ __device__ constexpr int adaptive_lanes(int nrows)

@@ -112,3 +112,43 @@ def test_batch_neighbours_in_the_stream(flags):
         for k, g in enumerate(got):
             assert torch.equal(g, want[k % 6]), f"run {k}"
     b.synchronize()
+
+
+@pytest.mark.parametrize("name,fmt,method", FORMATS)
+def test_event_between_streams(name, fmt, method):
+    """x is written late on another stream and handed over by an event; that stream overwrites
+    it as soon as an event says the product is done."""
+    case = CASES[name]
+    n = case[0]
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    hd = Handle(Cocktail.single(fmt, coo_of(case), method))
+    hd.set_stream(b.cuda_stream)
+    x, y = _view(hd, hd.vec_ptr, n), _view(hd, hd.res_ptr, n)
+    src = torch.rand(n, device="cuda") - 0.5
+    torch.cuda.synchronize()
+    outs = []
+    for late in (False, True):
+        got = []
+        for k in range(6):
+            with torch.cuda.stream(a):
+                if late:
+                    torch.cuda._sleep(200_000)
+                x.copy_(src * (k + 1))
+                written = torch.cuda.Event()
+                written.record(a)
+            with torch.cuda.stream(b):
+                y.zero_()
+                b.wait_event(written)
+                hd.do_spmv(1)
+                read = torch.cuda.Event()
+                read.record(b)
+                got.append(y.clone())
+            with torch.cuda.stream(a):
+                a.wait_event(read)
+                x.fill_(float("nan"))
+            if not late:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        outs.append(got)
+    for k, (p, q) in enumerate(zip(*outs)):
+        assert torch.isfinite(q).all() and torch.equal(p, q), f"round {k}"

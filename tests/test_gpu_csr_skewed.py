@@ -21,13 +21,14 @@ def _rows(lens, w, seed):
 
 
 CASES = {
-    # 256 rows a block: one lane a row, threshold 16
+    # 256 rows a block: one lane a row, threshold 32
     "at_16": _rows([16] * 100 + [17] + [1] * 300, 4000, 1),
+    "at_32": _rows([32] * 40 + [33] + [1] * 300 + [32, 33, 34] + [2] * 200, 4000, 8),
     "one_long": _rows([1] * 128 + [1700] + [1] * 127 + [0] * 300, 4000, 2),
     "many_long": _rows(([2] * 20 + [130, 0, 17]) * 30, 4000, 3),
-    # 2, 4, 8, 16, 32 lanes a row: thresholds 32 .. 512
-    "two_lanes": _rows(([14] * 100 + [33, 32, 500]) * 6, 4000, 4),
-    "eight_lanes": _rows(([60] * 20 + [129, 128, 400]) * 8, 4000, 5),
+    # 2, 4, 8, 16, 32 lanes a row: thresholds 64 .. 1024
+    "two_lanes": _rows(([14] * 100 + [33, 65, 64, 500]) * 6, 4000, 4),
+    "eight_lanes": _rows(([60] * 20 + [129, 257, 256, 400]) * 8, 4000, 5),
     "wide_rows": _rows([500, 600, 900] * 5 + [2040, 2041, 1, 3900, 0, 513, 512, 1015], 4000, 6),
     "zipf": M.zipf_rows(20_000, seed=7, max_len=3000),
 }
