@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) abar_dia_kernel(const int* __restrict__ o
 // shared memory.
 __global__ void __launch_bounds__(256) abar_dia4_kernel(const int* __restrict__ off, int nd, int len, int m, int n,
                                                         const float* ybar, const float* x,
-                                                        float* __restrict__ abar, bool beside)
+                                                        float* abar, bool beside)
 {
     extern __shared__ int s_off[];
     for (int i = threadIdx.x; i < nd; i += blockDim.x) s_off[i] = __ldg(off + i);
@@ -102,8 +102,7 @@ __global__ void __launch_bounds__(256) abar_dia4_kernel(const int* __restrict__ 
 // slot maps, row -1 on padding slots).
 __global__ void __launch_bounds__(256) abar_list_kernel(const int* __restrict__ rows, const int* __restrict__ cols,
                                                         size_t nslots, const float* ybar,
-                                                        const float* x, float* __restrict__ abar,
-                                                        int* __restrict__ prow, int* __restrict__ pcol, bool beside)
+                                                        const float* x, float* abar, int* prow, int* pcol, bool beside)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int r = i < nslots ? __ldg(rows + i) : -1, c = i < nslots ? __ldg(cols + i) : 0;

@@ -470,8 +470,7 @@ __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async
 template <class V>
 __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPart* __restrict__ parts,
                                                                   const BatchItem* __restrict__ items, int nitems, int fours,
-                                                                  int* __restrict__ next,
-                                                                  unsigned long long* __restrict__ cycles)
+                                                                  int* next, unsigned long long* cycles)
 {
     __shared__ __align__(16) BatchSmem sm;
     const int lane = threadIdx.x & 31;

@@ -197,7 +197,7 @@ __device__ __forceinline__ void gb_rows(const int* s_rp, const float* prod, cons
 template <class V, int BH, int BW>
 __global__ void __launch_bounds__(kGbThreads) bcsr_adaptive_kernel(const int* __restrict__ rp, const int* __restrict__ col,
                                                                    const V* __restrict__ data, const float* x,
-                                                                   float* __restrict__ y, const int4* __restrict__ work,
+                                                                   float* y, const int4* __restrict__ work,
                                                                    const unsigned short* __restrict__ tgt, int aligned, int m,
                                                                    int n)
 {

@@ -91,7 +91,7 @@ __device__ __forceinline__ float segment_dot(const int* __restrict__ col, const 
 template <class V, int G>
 __global__ void __launch_bounds__(256) csr_vector_kernel(const int* __restrict__ rp, const int* __restrict__ col,
                                                          const V* __restrict__ val, const float* x,
-                                                         float* __restrict__ y, int m)
+                                                         float* y, int m)
 {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int row = (int)(gid / G);
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kAdaptThreads) csr_adaptive_kernel(const int* 
                                                                      const float* yin, float* yout,
                                                                      const int4* __restrict__ blocks,
                                                                      const int4* __restrict__ long_rows,
-                                                                     float* __restrict__ partial, int* __restrict__ arrivals)
+                                                                     float* partial, int* arrivals)
 {
     __shared__ __align__(16) float prod[4 * kAdaptVecs];
     __shared__ int s_rp[kAdaptThreads + 1];
@@ -305,9 +305,9 @@ constexpr int kCooChunk = 128 * kCooTiles;
 template <class V>
 __global__ void __launch_bounds__(256) coo_segment_kernel(const int* __restrict__ rowid, const int* __restrict__ colid,
                                                           const V* __restrict__ val, const float* x,
-                                                          float* __restrict__ y, int nnz_pad, int nwarps,
+                                                          float* y, int nnz_pad, int nwarps,
                                                           const int* __restrict__ span_of_head, const int4* __restrict__ spans,
-                                                          int* __restrict__ span_count, float* __restrict__ part_val)
+                                                          int* span_count, float* part_val)
 {
     const int lane = threadIdx.x & 31;
     const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);

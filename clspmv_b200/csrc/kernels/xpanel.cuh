@@ -114,8 +114,7 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpanel_kernel(const int* __rest
                                                                const int* __restrict__ slot,
                                                                const unsigned short* __restrict__ lcol,
                                                                const V* __restrict__ val, const float* x,
-                                                               int n, int panel_w, float* __restrict__ partial,
-                                                               float* __restrict__ y)
+                                                               int n, int panel_w, float* partial, float* y)
 {
     extern __shared__ __align__(16) unsigned char xp_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -213,7 +212,7 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpanel_kernel(const int* __rest
 // over that row's slots and reducing with a fixed shuffle tree.
 __global__ void __launch_bounds__(256) xpanel_merge_kernel(const int* __restrict__ run_ptr, const int* __restrict__ run_rows,
                                                            int nrows, const int* __restrict__ long_list, int nlong,
-                                                           const float* __restrict__ partial, float* __restrict__ y)
+                                                           const float* partial, float* y)
 {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long short_threads = (long long)(nrows + 255) / 256 * 256;

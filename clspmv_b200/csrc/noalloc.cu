@@ -74,7 +74,7 @@ struct Tile {
 // chunk's first and last row go to the scratch pairs.
 __global__ void __launch_bounds__(256) coo_noalloc_segment(const int* rowid, const int* colid, const float* val, const float* x,
                                                            float* y, int nnz, int height, int width, int nwarps, int chunk,
-                                                           int* __restrict__ part_row, float* __restrict__ part_val)
+                                                           int* part_row, float* part_val)
 {
     dev::grid_dependency();   // the caller's arrays may be written by the operation before
     const int lane = threadIdx.x & 31;
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) coo_noalloc_segment(const int* rowid, con
 // followed through the next pairs 32 at a time (a row of 10,000 entries has 40 pairs: one
 // thread per run read them one after the other, 8 us of a 300,007-row Zipf product).  Runs
 // that start in an earlier warp's pairs are that warp's.
-__global__ void __launch_bounds__(256) coo_noalloc_fixup(const int* __restrict__ part_row, const float* __restrict__ part_val,
+__global__ void __launch_bounds__(256) coo_noalloc_fixup(const int* part_row, const float* part_val,
                                                          int nparts, int height, float* y)
 {
     const int i = blockIdx.x * 256 + threadIdx.x;
