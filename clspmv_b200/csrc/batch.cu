@@ -980,12 +980,14 @@ int csp_batch_create(const coo_matrix_if* const* mats, int n, const csp_batch_op
     }
     b->dparts = reinterpret_cast<dev::BatchPart*>(base + o_parts);
     BCUDA(cudaMemcpy(b->dparts, b->hparts.data(), b->hparts.size() * sizeof(dev::BatchPart), cudaMemcpyHostToDevice));
-    BCUDA(cudaMemset(b->counter, 0, 2 * sizeof(int)));
     for (int w : whats) {
         b->ditems[w] = reinterpret_cast<dev::BatchItem*>(base + o_items[w]);
         b->grid[w] = occupancy_grid(b->bf16, std::max(1, b->nitems[w]));
         b->fours[w] = leading_fours(b->ngathers[w], b->nitems[w] - b->ngathers[w], b->grid[w]);
     }
+    // the arena was cleared (the item counters with it) and filled on the legacy stream; the
+    // batch runs on streams that nothing orders behind it
+    BCUDA(cudaStreamSynchronize(cudaStreamLegacy));
     *out = b.release();
     return CSP_OK;
 }
