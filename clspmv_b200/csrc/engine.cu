@@ -15,6 +15,7 @@
 #include <limits.h>
 #include <string.h>
 #include <algorithm>
+#include <type_traits>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -668,6 +669,57 @@ int Engine::upload_block_records(Part& p, const bcsr_matrix_if& b)
     return e == cudaSuccess ? CSP_OK : cuda_error(e, "block records");
 }
 
+// f(SpmmShape) for a block shape and k right-hand sides: all float4 columns of k up to 32 in
+// one pass, so A is read once.
+template <class V, class F>
+static void with_spmm_shape(int bs, int k, F f)
+{
+    auto cols = [&](auto b) {
+        constexpr int B = decltype(b)::value;
+        if (k > 16) f(dev::SpmmShape<V, B, B, 8>{});
+        else if (k > 8) f(dev::SpmmShape<V, B, B, 4>{});
+        else if (k > 4) f(dev::SpmmShape<V, B, B, 2>{});
+        else f(dev::SpmmShape<V, B, B, 1>{});
+    };
+    switch (bs) {
+    case 1: cols(std::integral_constant<int, 1>{}); break;
+    case 2: cols(std::integral_constant<int, 2>{}); break;
+    case 3: cols(std::integral_constant<int, 3>{}); break;
+    case 4: cols(std::integral_constant<int, 4>{}); break;
+    case 6: cols(std::integral_constant<int, 6>{}); break;
+    }
+}
+
+// The block rows cut into the groups that one lane group of the SpMM kernel takes in turn: as
+// many consecutive rows as one wave of resident groups needs, up to max_rows (20,000 block
+// rows at k = 20 in 1.06 waves of 4 rows take 27.0 us, in one wave of 5 rows 22.9), but no
+// second row once a group would hold more than twice the mean's blocks: neighbouring long
+// rows are summed side by side, each by its own group (8 neighbours of 20,000 3x3 blocks among
+// 50,000 rows of 2 to 8, k = 32, one B200: 8.36 ms with eight rows a group, 1.07 so).
+int Engine::upload_spmm_groups(Part& p, const int* rp)
+{
+    int wave = 1, max_rows = 1;
+    auto shape = [&](auto sh) {
+        using Sh = decltype(sh);
+        wave = 148 * Sh::ctas * Sh::warps * Sh::groups;
+        max_rows = Sh::max_rows;
+    };
+    if (bf16) with_spmm_shape<__nv_bfloat16>(p.bh, nrhs, shape);
+    else with_spmm_shape<float>(p.bh, nrhs, shape);
+    const int nbr = p.nbr, rows = std::min(max_rows, (nbr + wave - 1) / wave);
+    const long long cap = nbr ? 2LL * rows * ((rp[nbr] - (long long)rp[0] + nbr - 1) / nbr) : 0;
+    std::vector<int4> g;
+    for (int r0 = 0, r1; r0 < nbr; r0 = r1) {
+        for (r1 = r0 + 1; r1 < nbr && r1 - r0 < rows && rp[r1 + 1] - (long long)rp[r0] <= cap;) r1++;
+        g.push_back(make_int4(r0, r1, rp[r0], rp[r1]));
+    }
+    p.nsgroups = (int)g.size();
+    int rc = alloc(reinterpret_cast<void**>(&p.sgroups), g.size() * sizeof(int4));
+    if (rc) return rc;
+    if (!g.empty()) CSP_CUDA(cudaMemcpy(p.sgroups, g.data(), g.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    return CSP_OK;
+}
+
 int Engine::add_generic_bcsr(const bcsr_matrix_if& b, int method)
 {
     const unsigned bw = b.bcsr_bwidth, bh = b.bcsr_bheight;
@@ -711,7 +763,7 @@ int Engine::add_generic_bcsr(const bcsr_matrix_if& b, int method)
     if (nrhs % 4 == 0 && !(tensor_spmm && nrhs % 32 == 0 && bw * bh <= 16) && (long long)width * (nrhs / 4) <= UINT32_MAX) {
         // several right-hand sides in whole float4s, X rows indexed in 32 bits: block records
         // (kernels/spmm.cuh)
-        if ((rc = upload_block_records(p, b))) return rc;
+        if ((rc = upload_block_records(p, b)) || (rc = upload_spmm_groups(p, b.bcsr_row_ptr))) return rc;
     } else if (!fits) {
         if ((rc = upload_int(&p.i1, b.bcsr_col_id, nblk, (size_t)pad_to(nblk, 4) + 4)) ||
             (rc = upload_val(&p.v, b.bcsr_data, nd, nd)))
@@ -798,33 +850,22 @@ static void launch_spmm(const Part& p, const float* x, float* y, int n, int k, b
     } else if (p.kind == PART_GBCSR && p.records) {
         const unsigned* rec = static_cast<const unsigned*>(p.v);
         if (p.nbr == 0) return;
-        // float4 columns per pass: all of k up to 32, so A is read once
-        const int CW = k > 16 ? 8 : (k > 8 ? 4 : (k > 4 ? 2 : 1));
-#define CSP_GB4K(BH, BW, C, K)                                                                                                   \
-    do {                                                                                                                         \
-        using Sh = SpmmShape<V, BH, BW, C>;                                                                                      \
-        /* as many block rows per lane group as one wave of resident groups needs, up to max_rows: */                            \
-        /* 20,000 block rows at k = 20 in 1.06 waves of 4 rows take 27.0 us, in one wave of 5 rows 22.9 */                          \
-        const int wave = 148 * Sh::ctas * Sh::warps * Sh::groups;                                                                \
-        const int rows = std::min(Sh::max_rows, (p.nbr + wave - 1) / wave);                                                      \
-        const long long ng = ((long long)p.nbr + rows - 1) / rows;                                                               \
-        launch_chained(bcsr_spmm_stream_kernel<V, BH, BW, C, K>, grid_for(ng * Sh::GL, Sh::threads), Sh::threads, 0, st,         \
-                       p.i0, rec, x, y, p.nbr, p.m, k, rows);                                                                    \
-    } while (0)
-#define CSP_GB4(BH, BW)                                                                                                          \
-    do {                                                                                                                         \
-        if (CW == 1) CSP_GB4K(BH, BW, 1, 4);                                                                                     \
-        else if (CW == 2) CSP_GB4K(BH, BW, 2, 8);                                                                                \
-        else if (CW == 4) CSP_GB4K(BH, BW, 4, 0);                                                                                \
-        else if (k == 32) CSP_GB4K(BH, BW, 8, 32);                                                                               \
-        else CSP_GB4K(BH, BW, 8, 0);                                                                                             \
-    } while (0)
-        switch (p.bh * 10 + p.bw) {
-        case 11: CSP_GB4(1, 1); break; case 22: CSP_GB4(2, 2); break; case 33: CSP_GB4(3, 3); break;
-        case 44: CSP_GB4(4, 4); break; case 66: CSP_GB4(6, 6); break;
-        }
-#undef CSP_GB4
-#undef CSP_GB4K
+        with_spmm_shape<V>(p.bh, k, [&](auto sh) {
+            using Sh = decltype(sh);
+            const unsigned g = grid_for((long long)p.nsgroups * Sh::GL, Sh::threads);
+            auto launch = [&](auto kc) {
+                launch_chained(bcsr_spmm_stream_kernel<V, Sh::BH, Sh::BW, Sh::CW, decltype(kc)::value>, g, Sh::threads, 0, st, p.sgroups,
+                               p.nsgroups, p.i0, rec, x, y, p.m, k);
+            };
+            if constexpr (Sh::CW <= 2) {
+                launch(std::integral_constant<int, 4 * Sh::CW>{});   // k is 4 or 8 here
+            } else if constexpr (Sh::CW == 8) {
+                if (k == 32) launch(std::integral_constant<int, 32>{});
+                else launch(std::integral_constant<int, 0>{});
+            } else {
+                launch(std::integral_constant<int, 0>{});
+            }
+        });
     } else if (p.kind == PART_GBCSR) {
         if (p.nbr == 0) return;
         const unsigned g = grid_for((long long)p.nbr * G, kSpmmThreads);

@@ -41,6 +41,8 @@ struct Part {
     int group = 0;    // CSR sub-warp lanes per row
     int nblocks = 0;  // CSR adaptive row blocks
     bool records = false;  // generic BCSR, k % 4 == 0: v holds block records (kernels/spmm.cuh)
+    int4* sgroups = nullptr;        // their groups of block rows {first, end, first block, end block}
+    int nsgroups = 0;
     int npad = 0, nwarps = 0;  // COO
     // x-panel layout (kernels/xpanel.cuh): i0 = run slot per entry, v = values
     unsigned short* lcol = nullptr;   // column inside the entry's panel
@@ -130,6 +132,7 @@ struct Engine {
     int add_sbell(const sbell_matrix_if& s, int method);
     int add_bcsr(const b4csr_matrix_if& b, int method);
     int upload_block_records(Part& p, const bcsr_matrix_if& b);
+    int upload_spmm_groups(Part& p, const int* rp);
     int add_generic_bcsr(const bcsr_matrix_if& b, int method);
 };
 

@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(kSpmmThreads) bcsr_spmm_kernel(const int* __re
 // Generic BCSR with k a multiple of 4, on a layout of its own: block j is BlockRec<V, BS>
 // words -- its BS values in row-major order (two per word in BF16), then the index of
 // its first X row in float4s -- so a run of blocks is one contiguous stream.  A warp is
-// cut into groups of GL = 4 CW lanes; a group takes `rows` consecutive block rows one
-// after the other and copies their blocks through a ring of four chunks in shared memory
+// cut into groups of GL = 4 CW lanes; a group takes consecutive block rows (the host's
+// `groups`: at most max_rows, and at most one where a row is long) one after the other and copies their blocks through a ring of four chunks in shared memory
 // with 16-byte cp.async, two chunks ahead.  Per step a group takes 4 U blocks of its
 // current row: lane (cw, sub) owns right-hand sides 4 cw .. 4 cw + 3 of blocks sub,
 // sub + 4, ..., whose X loads are all in flight together.  At the end of a row the four
@@ -200,8 +200,8 @@ __device__ __forceinline__ void read_block(const unsigned* s, float (&a)[BS])
 }
 
 // The lane split for CW float4 columns a pass.
-template <class V, int BH, int BW, int CW> struct SpmmShape {
-    static constexpr int BS = BH * BW;
+template <class V, int BH_, int BW_, int CW_> struct SpmmShape {
+    static constexpr int BH = BH_, BW = BW_, CW = CW_, BS = BH * BW;
     static constexpr int GL = 4 * CW, groups = 32 / GL;
     // rounds of X loads in flight: two, where 64 registers hold them; at one float4 column
     // (k = 4) one, which halves the ring and keeps more warps resident (197 -> 182 us)
@@ -211,7 +211,7 @@ template <class V, int BH, int BW, int CW> struct SpmmShape {
     static constexpr int warp_bytes = groups * ring_words * 4;
     static constexpr int warps = warp_bytes * 8 <= 48 * 1024 ? 8 : (warp_bytes * 4 <= 48 * 1024 ? 4 : (warp_bytes * 2 <= 48 * 1024 ? 2 : 1));
     static constexpr int threads = 32 * warps;
-    // consecutive block rows per group: a warp per row needs eight to hide the start of its ring
+    // consecutive block rows per group, at most: a warp per row needs eight to hide the start of its ring
     static constexpr int max_rows = groups == 1 ? 8 : 4;
     static constexpr int ctas = (BS <= 9 ? 32 : (BS <= 16 ? 24 : 16)) / warps;   // per SM
 };
@@ -219,7 +219,8 @@ template <class V, int BH, int BW, int CW> struct SpmmShape {
 // K: the number of right-hand sides where it is known (0: `k_arg`).
 template <class V, int BH, int BW, int CW, int K>
 __global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V, BH, BW, CW>::ctas)
-    bcsr_spmm_stream_kernel(const int* __restrict__ rp, const unsigned* __restrict__ rec, const float* x, float* y, int nbr, int m, int k_arg, int rows)
+    bcsr_spmm_stream_kernel(const int4* __restrict__ groups, int ngroups, const int* __restrict__ rp, const unsigned* __restrict__ rec,
+                            const float* x, float* y, int m, int k_arg)
 {
     using Sh = SpmmShape<V, BH, BW, CW>;
     using Rec = BlockRec<V, BH * BW>;
@@ -232,10 +233,11 @@ __global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V
     unsigned* ring = s_ring[threadIdx.x / GL];
     const unsigned ring_addr = (unsigned)__cvta_generic_to_shared(ring);
     const int gid = (int)(((long long)blockIdx.x * Sh::threads + threadIdx.x) / GL);
-    const int r0 = (int)min((long long)gid * rows, (long long)nbr), r1 = min(r0 + rows, nbr);
+    // block rows [x, y) with blocks [z, w)
+    const int4 gr = gid < ngroups ? __ldg(groups + gid) : make_int4(0, 0, 0, 0);
+    const int r0 = gr.x, r1 = gr.y, sb = gr.z, eb = gr.w;
     const int cw = lane % CW, sub = lane / CW;
     const int rend = __ldg(rp + min(r0 + 1 + lane, r1));     // rows <= GL: the ends of the group's rows
-    const int sb = __ldg(rp + r0), eb = __ldg(rp + r1);
     const int base = sb & ~1;                                // chunks start on 16 bytes
     // the right-hand side of this lane's results: c + comp
     const int comp = ((lane & CW) ? 2 : 0) + ((lane & (2 * CW)) ? 1 : 0);
