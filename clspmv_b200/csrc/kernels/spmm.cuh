@@ -213,7 +213,10 @@ template <class V, int BH_, int BW_, int CW_> struct SpmmShape {
     static constexpr int threads = 32 * warps;
     // consecutive block rows per group, at most: a warp per row needs eight to hide the start of its ring
     static constexpr int max_rows = groups == 1 ? 8 : 4;
-    static constexpr int ctas = (BS <= 9 ? 32 : (BS <= 16 ? 24 : 16)) / warps;   // per SM
+    // per SM: by registers, and by the rings in its 228 KB of shared memory (1 KB a CTA is the system's)
+    static constexpr int reg_ctas = (BS <= 9 ? 32 : (BS <= 16 ? 24 : 16)) / warps;
+    static constexpr int smem_ctas = 228 * 1024 / (warps * warp_bytes + 1024);
+    static constexpr int ctas = reg_ctas < smem_ctas ? reg_ctas : smem_ctas;
 };
 
 // K: the number of right-hand sides where it is known (0: `k_arg`).
@@ -227,6 +230,7 @@ __global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V
     constexpr int BS = BH * BW, GL = Sh::GL, U = Sh::U, CH = Sh::chunk, NW = Rec::words;
     constexpr int RM = 4 * CH - 1;   // ring index mask
     static_assert((CH & (CH - 1)) == 0 && CH * NW % 4 == 0, "ring of a power of two blocks, whole 16-byte copies");
+    static_assert(Sh::ctas >= 1 && Sh::ctas * (Sh::warps * Sh::warp_bytes + 1024) <= 228 * 1024, "the CTAs that a wave counts on fit an SM");
     __shared__ __align__(16) unsigned s_ring[32 * Sh::warps / GL][Sh::ring_words];
     const int k = K ? K : k_arg;
     const int lane = threadIdx.x % GL;                       // in the group
