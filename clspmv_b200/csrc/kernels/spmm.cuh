@@ -204,8 +204,11 @@ template <class V, int BH_, int BW_, int CW_> struct SpmmShape {
     static constexpr int BH = BH_, BW = BW_, CW = CW_, BS = BH * BW;
     static constexpr int GL = 4 * CW, groups = 32 / GL;
     // rounds of X loads in flight: two, where 64 registers hold them; at one float4 column
-    // (k = 4) one, which halves the ring and keeps more warps resident (197 -> 182 us)
-    static constexpr int U = BW > 4 || CW == 1 ? 1 : 2;
+    // (k = 4) one for 3x3 and 4x4, which halves the ring and keeps more warps resident (197 ->
+    // 182 us); for 1x1, whose rounds are one load a lane, four (100,000 rows of 10 to 30 entries,
+    // one B200, before -> with four: k = 4 24.3 -> 17.1 us, k = 32 31.0 -> 29.3; 120,000 Zipf rows,
+    // k = 4 420 -> 118).  2x2, k = 4, 30,000 block rows: one 13.0, two 10.5
+    static constexpr int U = BW == 1 ? 4 : (BW > 4 || (BW > 2 && CW == 1) ? 1 : 2);
     static constexpr int chunk = 4 * U > 2 * CW ? 4 * U : 2 * CW;               // blocks; a step spans at most two
     static constexpr int ring_words = 4 * chunk * BlockRec<V, BS>::words;       // per group
     static constexpr int warp_bytes = groups * ring_words * 4;

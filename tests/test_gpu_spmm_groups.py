@@ -77,8 +77,8 @@ def test_row_groups(bs, k, most, bf16):
         assert err <= TOL, f"column {j}: error {err:.3e} at row {row}"
 
 
-def _time_us(degs, k):
-    b, (h, w, *_) = _bcsr(degs, 3, 3, nbc=20_000)
+def _time_us(degs, k, bs=3):
+    b, (h, w, *_) = _bcsr(degs, bs, 3, nbc=20_000)
     hd = Handle(None, np.ones((w, k), np.float32), None, nrhs=k, bcsr=b)
     st = torch.cuda.Stream()
     hd.set_stream(st.cuda_stream)
@@ -107,3 +107,11 @@ def test_neighbouring_long_rows(k):
     far[3_000::6_000][:8] = 10_000
     assert near.sum() == far.sum()
     assert _time_us(near, k) <= 2 * _time_us(far, k)
+
+
+def test_long_row_of_single_entries():
+    """A row of 20,000 1x1 blocks at 4 right-hand sides has as many loads in flight as at 32, so it
+    takes no longer (with one load a lane in flight it took 2.4 times as long)."""
+    d = np.full(50_000, 3)
+    d[::10_000] = 20_000
+    assert _time_us(d, 4, bs=1) <= 1.6 * _time_us(d, 32, bs=1)
