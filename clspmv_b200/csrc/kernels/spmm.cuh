@@ -216,8 +216,10 @@ template <class V, int BH_, int BW_, int CW_> struct SpmmShape {
     static constexpr int threads = 32 * warps;
     // consecutive block rows per group, at most: a warp per row needs eight to hide the start of its ring
     static constexpr int max_rows = groups == 1 ? 8 : 4;
-    // per SM: by registers, and by the rings in its 228 KB of shared memory (1 KB a CTA is the system's)
-    static constexpr int reg_ctas = (BS <= 9 ? 32 : (BS <= 16 ? 24 : 16)) / warps;
+    // per SM: by registers, and by the rings in its 228 KB of shared memory (1 KB a CTA is the system's).
+    // 4x4 blocks and larger at 16 warps (128 registers): at 24 the 4x4 FP32 kernel that takes any k had no
+    // room for its X loads (30,000 block rows, one B200: k = 64 112 -> 91.6 us, k = 20 51.8 -> 43.7)
+    static constexpr int reg_ctas = (BS <= 9 ? 32 : 16) / warps;
     static constexpr int smem_ctas = 228 * 1024 / (warps * warp_bytes + 1024);
     static constexpr int ctas = reg_ctas < smem_ctas ? reg_ctas : smem_ctas;
 };

@@ -115,3 +115,10 @@ def test_long_row_of_single_entries():
     d = np.full(50_000, 3)
     d[::10_000] = 20_000
     assert _time_us(d, 4, bs=1) <= 1.6 * _time_us(d, 32, bs=1)
+
+
+def test_two_passes_cost_twice_one():
+    """4x4 blocks at k = 64 are two passes of the kernel at k = 32 (with 24 warps an SM they took
+    2.4 times as long, the kernel that takes any k being short of registers)."""
+    d = np.random.default_rng(5).integers(10, 31, 30_000)
+    assert _time_us(d, 64, bs=4) <= 2.25 * _time_us(d, 32, bs=4)
