@@ -457,8 +457,13 @@ __global__ void __launch_bounds__(256) ell_kernel(const int* __restrict__ col, c
 }
 
 // ELL, four consecutive rows per thread with 128-bit loads (spmv_ell.cl gpu_ell_v4;
-// height_aligned is a multiple of 4): yout = yin + A x.  The columns and values of
-// kEllAhead slots are requested together, the first ones before grid_dependency().
+// height_aligned is a multiple of 4): yout = yin + A x.  The columns and values of the first
+// kEllAhead slots are requested together, before grid_dependency(); the slots past them go
+// through a plain loop, whose loads of up to four slots the compiler keeps in flight.  Random
+// gathers bound it: a test of the slot between them (as in a loop over batches of kEllAhead
+// whose last one is short) leaves one slot in flight.  50,000 rows of 40 slots, one B200: 23.3 us
+// so, 10.5 without it (14.4 before slots were requested ahead); 20,000 rows of 300: 94.9, 52.3
+// (61.9); unrolled by eight the loop takes 9.0 us instead of 7.6 on 500,000 rows of 12 near slots.
 constexpr int kEllAhead = 5;
 
 template <class V>
@@ -467,33 +472,37 @@ __global__ void __launch_bounds__(256) ell_rows_kernel(const int* __restrict__ c
 {
     const int r0 = (blockIdx.x * 256 + threadIdx.x) * 4;
     if (r0 >= m) return;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](int4 c, float4 a) {
+        acc.x += a.x * x[c.x];
+        acc.y += a.y * x[c.y];
+        acc.z += a.z * x[c.z];
+        acc.w += a.w * x[c.w];
+    };
     int4 c[kEllAhead];
     float4 a[kEllAhead];
-    auto fetch = [&](int k0) {
 #pragma unroll
-        for (int u = 0; u < kEllAhead; u++)
-            if (k0 + u < ell_num) {
-                const size_t j = (size_t)(k0 + u) * hal + r0;
-                c[u] = ld_int4(col + j);
-                a[u] = Val<V>::ld4(val + j);
-            }
-    };
-    fetch(0);
+    for (int u = 0; u < kEllAhead; u++)
+        if (u < ell_num) {
+            const size_t j = (size_t)u * hal + r0;
+            c[u] = ld_int4(col + j);
+            a[u] = Val<V>::ld4(val + j);
+        }
     grid_dependency();
     float yo[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) yo[q] = r0 + q < m ? yin[r0 + q] : 0.0f;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < ell_num; k += kEllAhead) {
-        if (k) fetch(k);
+    if (ell_num >= kEllAhead) {   // no test between the gathers
 #pragma unroll
-        for (int u = 0; u < kEllAhead; u++) {
-            if (k + u >= ell_num) break;
-            acc.x += a[u].x * x[c[u].x];
-            acc.y += a[u].y * x[c[u].y];
-            acc.z += a[u].z * x[c[u].z];
-            acc.w += a[u].w * x[c[u].w];
-        }
+        for (int u = 0; u < kEllAhead; u++) add(c[u], a[u]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < kEllAhead; u++)
+            if (u < ell_num) add(c[u], a[u]);
+    }
+    for (int k = kEllAhead; k < ell_num; k++) {
+        const size_t j = (size_t)k * hal + r0;
+        add(ld_int4(col + j), Val<V>::ld4(val + j));
     }
     yout[r0] = yo[0] + acc.x;
     if (r0 + 1 < m) yout[r0 + 1] = yo[1] + acc.y;
