@@ -37,6 +37,7 @@ struct Part {
     int maxw = 0;     // BDIA widest band
     int2* dgroups = nullptr;        // DIA, BDIA: groups of consecutive offsets {first offset, diagonals}
     int ngroups = 0;
+    bool alone = false;             // every group is one diagonal (dia_each_kernel)
     int off_min = 0, off_max = 0;   // smallest and largest offset
     int group = 0;    // CSR sub-warp lanes per row
     int nblocks = 0;  // CSR adaptive row blocks
