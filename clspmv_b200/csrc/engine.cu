@@ -514,9 +514,21 @@ int Engine::add_dia(const dia_matrix_iif& d)
     return CSP_OK;
 }
 
+// Wide BF16 bands that stay in L2 run the staged kernel: dia_rows_kernel copies them in pieces of
+// 8 bytes, which bounds it where DRAM does not.  One B200, staged / rows: one band of 64 on 600,000 rows
+// 17.9 / 22.1 us, two of 24 14.4 / 16.4, one of 256 on 50,000 33.0 / 37.8, of 128 on 200,000 20.2 / 22.2.
+// Smaller matrices and narrower bands (48 on 200,000 rows 10.3 / 9.0, 96 on 50,000 15.1 / 14.6), and
+// larger ones (256 on 200,000 rows, 102 MB, 80.3 / 43.9), are for the other, and so is FP32.
+static bool staged_bands(bool bf16, int bands, int ndia, int maxw, int len)
+{
+    const size_t bytes = (size_t)ndia * len * 2;
+    return bf16 && bands > 0 && ndia >= 24 * (long long)bands && maxw <= dev::kBdiaStagedMax && bytes <= (size_t)80 << 20 &&
+           (bytes >= (size_t)36 << 20 || ndia >= 112 * (long long)bands);
+}
+
 // Every BDIA method of the reference (spmv_cocktail.cpp:339-358: 0 nlvec, 1 staged, 2 staged
-// (g4), 3 v4_nlvec, 4 v4 staged) runs the four-row diagonal kernel over the bands' expanded
-// offsets; diagonals not aligned to four rows, the staged one.
+// (g4), 3 v4_nlvec, 4 v4 staged) runs the four-row diagonal kernels over the bands' expanded
+// offsets, or the staged one; diagonals not aligned to four rows always the staged one.
 int Engine::add_bdia(const bdia_matrix_iif& b)
 {
     const int len = b.bdia_length_aligned;
@@ -530,9 +542,10 @@ int Engine::add_bdia(const bdia_matrix_iif& b)
     int maxw = 1;
     for (int i = 0; i < b.bdia_band_num; i++) maxw = std::max(maxw, b.bdia_bptr[i + 1] - b.bdia_bptr[i]);
     p.maxw = maxw;
-    p.method = len % 4 == 0 ? 1 : 0;
+    p.method = len % 4 == 0 && !staged_bands(bf16, b.bdia_band_num, ndia, maxw, len) ? 1 : 0;
     // the staged kernel's window would not fit in shared memory
-    if (p.method == 0 && maxw > 8000) return set_error(CSP_EUNSUP, "BDIA part: band wider than 8000 with unaligned length");
+    if (p.method == 0 && maxw > dev::kBdiaStagedMax)
+        return set_error(CSP_EUNSUP, "BDIA part: band wider than %d with unaligned length", dev::kBdiaStagedMax);
     for (int i = 0; i < b.bdia_band_num; i++)
         if (b.bdia_bptr[i + 1] < b.bdia_bptr[i] || b.bdia_bptr[0] != 0) return set_error(CSP_EINVAL, "BDIA part: bad band pointer");
     const size_t n = (size_t)ndia * len;

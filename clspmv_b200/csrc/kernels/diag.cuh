@@ -233,6 +233,8 @@ __global__ void __launch_bounds__(kDiaThreads) dia_each_kernel(const int2* __res
         if (r0 + q < m) yout[r0 + q] = yo[q] + (q == 0 ? acc.x : q == 1 ? acc.y : q == 2 ? acc.z : acc.w);
 }
 
+constexpr int kBdiaStagedMax = 8000;   // widest band whose window fits 48 KB of shared memory
+
 // BDIA with the band's window of x staged in shared memory (spmv_bdia.cl gpu_bdia:
 // one staged window per band, reused by the band's adjacent diagonals).  The CTA
 // covers kDiaThreads*ROWS rows, thread t owning rows t, t+256, ... so shared-memory
