@@ -1224,7 +1224,7 @@ int Engine::set_l2_window()
     return CSP_OK;
 }
 
-int Engine::init_common(int w, int h, int nz, const float* vec, const float* res, int flags, int k)
+int Engine::init_common(int w, int h, int nz, int flags, int k)
 {
     width = w;
     height = h;
@@ -1244,13 +1244,19 @@ int Engine::init_common(int w, int h, int nz, const float* vec, const float* res
     // y: padded to a multiple of 1024 like the reference (spmv_cocktail.cpp:234)
     x_len = pad_to(std::max(width, 1), 64) + 64;
     y_len = pad_to(std::max(height, 1), 1024);
-    // a square matrix's x has room for csp_iterate's second vector behind it (one allocation:
-    // a second one adds 0.1-0.3 ms to the set-up)
-    const size_t x_floats = (size_t)x_len * nrhs * (width == height && nrhs == 1 ? 2 : 1);
+    return CSP_OK;
+}
+
+// x, y and, where csp_iterate's steps alternate (`steps`), its second vector behind x (in one
+// allocation: a second one adds 0.1-0.3 ms to the set-up).  Called once the parts are known.
+int Engine::init_vectors(const float* vec, const float* res, int flags, bool steps)
+{
+    const size_t x_floats = (size_t)x_len * nrhs * (steps ? 2 : 1);
     int rc;
     if ((rc = alloc(reinterpret_cast<void**>(&d_x), x_floats * 4)) ||
         (rc = alloc(reinterpret_cast<void**>(&d_y), (size_t)y_len * nrhs * 4)))
         return rc;
+    if (steps) d_z = d_x + x_len;
     CSP_CUDA(cudaMemset(d_x, 0, x_floats * 4));
     CSP_CUDA(cudaMemset(d_y, 0, (size_t)y_len * nrhs * 4));
     if (vec && width) CSP_CUDA(cudaMemcpy(d_x, vec, (size_t)width * nrhs * 4, cudaMemcpyHostToDevice));
@@ -1262,7 +1268,7 @@ int Engine::init_common(int w, int h, int nz, const float* vec, const float* res
 int Engine::init(const cocktail_iif* mat, const float* vec, const float* res, int flags, int k)
 {
     if (!mat) return set_error(CSP_EINVAL, "null cocktail");
-    int rc = init_common(mat->mat_width, mat->mat_height, mat->mat_nnz, vec, res, flags, k);
+    int rc = init_common(mat->mat_width, mat->mat_height, mat->mat_nnz, flags, k);
     if (rc) return rc;
     static_assert(sizeof(bcsr_matrix_if) == sizeof(b4csr_matrix_if) &&
                       offsetof(bcsr_matrix_if, bcsr_row_ptr) == offsetof(b4csr_matrix_if, b4csr_row_ptr) &&
@@ -1293,8 +1299,8 @@ int Engine::init(const cocktail_iif* mat, const float* vec, const float* res, in
     if (mat->ifusecsr && (rc = add_csr(mat->csr, mat->csr_meth_num))) return rc;
     if (mat->ifusecoo && (rc = add_coo(mat->coo, mat->coo_meth_num))) return rc;
     if ((flags & CSP_FLAG_ADJOINT) && (rc = build_adjoint(mat))) return rc;
-    if (width == height && nrhs == 1 && parts.size() == 1 && has_step(parts[0]) && parts[0].m == height && height > 0)
-        d_z = d_x + x_len;   // csp_iterate
+    const bool steps = width == height && nrhs == 1 && parts.size() == 1 && has_step(parts[0]) && parts[0].m == height && height > 0;
+    if ((rc = init_vectors(vec, res, flags, steps))) return rc;
     CSP_CUDA(cudaDeviceSynchronize());
     return CSP_OK;
 }
@@ -1304,10 +1310,11 @@ int Engine::init_bcsr(const bcsr_matrix_if* b, const float* vec, const float* re
     if (!b) return set_error(CSP_EINVAL, "null BCSR");
     if ((flags & CSP_FLAG_ADJOINT) && k > 1) return set_error(CSP_EUNSUP, "adjoint with several right-hand sides");
     if (k > 1 && b->bcsr_bwidth * b->bcsr_bheight > 36) return set_error(CSP_EUNSUP, "several right-hand sides need blocks of <= 36 elements");
-    int rc = init_common(b->matinfo.width, b->matinfo.height, b->matinfo.nnz, vec, res, flags, k);
+    int rc = init_common(b->matinfo.width, b->matinfo.height, b->matinfo.nnz, flags, k);
     if (rc) return rc;
     if ((rc = add_generic_bcsr(*b, 0))) return rc;
     if ((flags & CSP_FLAG_ADJOINT) && (rc = build_adjoint_gbcsr(*b))) return rc;
+    if ((rc = init_vectors(vec, res, flags, false))) return rc;
     CSP_CUDA(cudaDeviceSynchronize());
     return CSP_OK;
 }

@@ -101,7 +101,8 @@ struct Engine {
 
     ~Engine();
     int init(const cocktail_iif* mat, const float* vec, const float* res, int flags, int k = 1);
-    int init_common(int w, int h, int nz, const float* vec, const float* res, int flags, int k);
+    int init_common(int w, int h, int nz, int flags, int k);
+    int init_vectors(const float* vec, const float* res, int flags, bool steps);
     int init_bcsr(const bcsr_matrix_if* b, const float* vec, const float* res, int flags, int k);
     int spmv(int ntimes);
     int iterate(int iterations);
