@@ -42,7 +42,7 @@ def _chained():
     for path in sorted(glob.glob(os.path.join(CSRC, "kernels", "*.cuh")) + glob.glob(os.path.join(CSRC, "*.cu"))):
         with open(path) as f:
             for name, params, body in _kernels(f.read()):
-                if "grid_dependency(" in body or "gradient_begin(" in body:
+                if re.search(r"grid_dependency\w*\(|gradient_begin\(", body):
                     found[name] = [p.strip() for p in params.split(",") if "*" in p]
     return found
 
