@@ -163,9 +163,12 @@ constexpr int kGbRows = 128;
 
 // A CTA requests for L2 the blocks of the item half a wave of CTAs later (148 SMs x 8 CTAs), so
 // DRAM keeps working while the CTAs gather and reduce.  10 M 3x3 blocks, one B200, in a graph:
-// FP32 93.4 -> 86.3 us, BF16 80.9 -> 77.8; a quarter wave ahead 87.9, an eighth 92.7, one and a
-// half waves 89.9, two 94.5.
+// FP32 93.4 -> 86.3 us, BF16 80.9 -> 77.8 (beyond L2 with the L2 flushed before each call, as the
+// benchmark times it, 98.1 -> 94.1 and 86.0 -> 86.0); a quarter wave ahead 87.9, an eighth 92.7,
+// one and a half waves 89.9, two 94.5.  Not for 1x1 and FP32 2x2 blocks: 8 M 2x2 blocks take 48.2 us
+// without and 59.8 with it in FP32 (45.7 and 42.3 in BF16), 1x1 23.1 and 24.0.
 constexpr unsigned kGbAhead = 148 * 4;
+__host__ __device__ constexpr bool gb_ahead(int elements, int value_bytes) { return elements >= (value_bytes == 4 ? 9 : 4); }
 
 // Row sums of one item: a lane group of G lanes per block row adds the row's block
 // products (prod, row order) and writes y = s_y + sum (s_y: the item's y rows).
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(kGbThreads) bcsr_adaptive_kernel(const int* __
         for (int k = 0; k < BH * BW; k++) d[k] = Val<V>::ld4(data + (size_t)k * aligned + j);
     }
     // the blocks of the item kGbAhead CTAs on go to L2, a plane per lane of the last warp
-    if (tid >= kGbThreads - 32 && blockIdx.x + kGbAhead < gridDim.x) {
+    if (gb_ahead(BH * BW, sizeof(V)) && tid >= kGbThreads - 32 && blockIdx.x + kGbAhead < gridDim.x) {
         const int4 nw = __ldg(work + blockIdx.x + kGbAhead);
         const int l = tid - (kGbThreads - 32), slots = ((nw.y >> 16) + 3) & ~3;
         if (l < BH * BW) prefetch_l2(data + (size_t)l * aligned + nw.w, slots * (int)sizeof(V));
