@@ -927,8 +927,20 @@ static void launch_step(const Part& p, const float* x, const float* yin, float* 
     if (p.kind == PART_CSR)
         launch_chained(csr_adaptive_kernel<V>, p.nblocks, kAdaptThreads, 0, st, p.i0, p.i1, v, x, yin, yout, p.blocks, p.long_rows,
                p.scratch_val, p.scratch_row);
-    else if (p.kind == PART_ELL)
-        launch_chained(ell_rows_kernel<V>, grid_for((p.m + 3) / 4, 256), 256, 0, st, p.i1, v, x, yin, yout, p.m, p.k, p.stride);
+    else if (p.kind == PART_ELL) {
+        auto launch = [&](auto a) {
+            launch_chained(ell_rows_kernel<V, decltype(a)::value>, grid_for((p.m + 3) / 4, 256), 256, 0, st, p.i1, v, x, yin, yout, p.m, p.k,
+                           p.stride);
+        };
+        switch (std::min(p.k, kEllAhead)) {
+        case 0: launch(std::integral_constant<int, 0>{}); break;
+        case 1: launch(std::integral_constant<int, 1>{}); break;
+        case 2: launch(std::integral_constant<int, 2>{}); break;
+        case 3: launch(std::integral_constant<int, 3>{}); break;
+        case 4: launch(std::integral_constant<int, 4>{}); break;
+        default: launch(std::integral_constant<int, kEllAhead>{}); break;
+        }
+    }
     else if (p.alone)
         launch_chained(dia_each_kernel<V>, grid_for((p.m + 3) / 4, kDiaThreads), kDiaThreads, p.ngroups * sizeof(int), st, p.dgroups, v, x,
                        yin, yout, p.m, n, p.ngroups, p.stride);

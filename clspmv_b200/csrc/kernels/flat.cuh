@@ -457,16 +457,17 @@ __global__ void __launch_bounds__(256) ell_kernel(const int* __restrict__ col, c
 }
 
 // ELL, four consecutive rows per thread with 128-bit loads (spmv_ell.cl gpu_ell_v4;
-// height_aligned is a multiple of 4): yout = yin + A x.  The columns and values of the first
-// kEllAhead slots are requested together, before grid_dependency(); the slots past them go
-// through a plain loop, whose loads of up to four slots the compiler keeps in flight.  Random
-// gathers bound it: a test of the slot between them (as in a loop over batches of kEllAhead
-// whose last one is short) leaves one slot in flight.  50,000 rows of 40 slots, one B200: 23.3 us
-// so, 10.5 without it (14.4 before slots were requested ahead); 20,000 rows of 300: 94.9, 52.3
-// (61.9); unrolled by eight the loop takes 9.0 us instead of 7.6 on 500,000 rows of 12 near slots.
+// height_aligned is a multiple of 4): yout = yin + A x.  The columns and values of the first A
+// slots, A = min(ell_num, kEllAhead), are requested together, before grid_dependency(); the slots past
+// them go through a plain loop.  Random gathers bound it: a test of the slot between them (as in a
+// loop over batches whose last one is short) leaves one slot in flight.  50,000 rows of 40 slots, one
+// B200: 23.3 us so, 10.9 without it (14.4 before slots were requested ahead); 20,000 rows of 300: 94.9,
+// 49.4 (61.9; the loop unrolled by four 69).  One kernel for every A holds 76 registers where one slot
+// needs 32: 5 M rows of one slot 15.9 us so, 10.6 with a kernel for each A (14.4 before).
 constexpr int kEllAhead = 5;
 
-template <class V>
+// A: min(ell_num, kEllAhead)
+template <class V, int A>
 __global__ void __launch_bounds__(256) ell_rows_kernel(const int* __restrict__ col, const V* __restrict__ val, const float* x,
                                                        const float* yin, float* yout, int m, int ell_num, int hal)
 {
@@ -479,31 +480,26 @@ __global__ void __launch_bounds__(256) ell_rows_kernel(const int* __restrict__ c
         acc.z += a.z * x[c.z];
         acc.w += a.w * x[c.w];
     };
-    int4 c[kEllAhead];
-    float4 a[kEllAhead];
+    int4 c[A ? A : 1];
+    float4 a[A ? A : 1];
 #pragma unroll
-    for (int u = 0; u < kEllAhead; u++)
-        if (u < ell_num) {
-            const size_t j = (size_t)u * hal + r0;
-            c[u] = ld_int4(col + j);
-            a[u] = Val<V>::ld4(val + j);
-        }
+    for (int u = 0; u < A; u++) {
+        const size_t j = (size_t)u * hal + r0;
+        c[u] = ld_int4(col + j);
+        a[u] = Val<V>::ld4(val + j);
+    }
     grid_dependency();
     float yo[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) yo[q] = r0 + q < m ? yin[r0 + q] : 0.0f;
-    if (ell_num >= kEllAhead) {   // no test between the gathers
 #pragma unroll
-        for (int u = 0; u < kEllAhead; u++) add(c[u], a[u]);
-    } else {
-#pragma unroll
-        for (int u = 0; u < kEllAhead; u++)
-            if (u < ell_num) add(c[u], a[u]);
-    }
-    for (int k = kEllAhead; k < ell_num; k++) {
-        const size_t j = (size_t)k * hal + r0;
-        add(ld_int4(col + j), Val<V>::ld4(val + j));
-    }
+    for (int u = 0; u < A; u++) add(c[u], a[u]);
+    if (A == kEllAhead)
+#pragma unroll 6
+        for (int k = A; k < ell_num; k++) {
+            const size_t j = (size_t)k * hal + r0;
+            add(ld_int4(col + j), Val<V>::ld4(val + j));
+        }
     yout[r0] = yo[0] + acc.x;
     if (r0 + 1 < m) yout[r0 + 1] = yo[1] + acc.y;
     if (r0 + 2 < m) yout[r0 + 2] = yo[2] + acc.z;
