@@ -695,14 +695,20 @@ int Engine::upload_block_records(Part& p, const bcsr_matrix_if& b)
 // f(SpmmShape) for a block shape and k right-hand sides: all float4 columns of k up to 32 in
 // one pass, so A is read once.
 template <class V, class F>
-static void with_spmm_shape(int bs, int k, F f)
+static void with_spmm_shape(int bs, int k, bool many, F f)
 {
+    auto shape = [&](auto b, auto c) {
+        constexpr int B = decltype(b)::value, C = decltype(c)::value;
+        if constexpr (dev::spmm_has_many(B, C)) {
+            if (many) return f(dev::SpmmShape<V, B, B, C, true>{});
+        }
+        f(dev::SpmmShape<V, B, B, C>{});
+    };
     auto cols = [&](auto b) {
-        constexpr int B = decltype(b)::value;
-        if (k > 16) f(dev::SpmmShape<V, B, B, 8>{});
-        else if (k > 8) f(dev::SpmmShape<V, B, B, 4>{});
-        else if (k > 4) f(dev::SpmmShape<V, B, B, 2>{});
-        else f(dev::SpmmShape<V, B, B, 1>{});
+        if (k > 16) shape(b, std::integral_constant<int, 8>{});
+        else if (k > 8) shape(b, std::integral_constant<int, 4>{});
+        else if (k > 4) shape(b, std::integral_constant<int, 2>{});
+        else shape(b, std::integral_constant<int, 1>{});
     };
     switch (bs) {
     case 1: cols(std::integral_constant<int, 1>{}); break;
@@ -727,10 +733,16 @@ int Engine::upload_spmm_groups(Part& p, const int* rp)
         wave = 148 * Sh::ctas * Sh::warps * Sh::groups;
         max_rows = Sh::max_rows;
     };
-    if (bf16) with_spmm_shape<__nv_bfloat16>(p.bh, nrhs, shape);
-    else with_spmm_shape<float>(p.bh, nrhs, shape);
-    const int nbr = p.nbr, rows = std::min(max_rows, (nbr + wave - 1) / wave);
-    const long long cap = nbr ? 2LL * rows * ((rp[nbr] - (long long)rp[0] + nbr - 1) / nbr) : 0;
+    // rows of many blocks: by the mean, or by a longest row whose chain of rounds outlasts the others
+    const int nbr = p.nbr;
+    const long long nblk = nbr ? rp[nbr] - (long long)rp[0] : 0;
+    int longest = 0;
+    for (int r = 0; r < nbr; r++) longest = std::max(longest, rp[r + 1] - rp[r]);
+    p.many = nblk >= 9LL * nbr || longest >= std::max(64, nbr / 64);
+    if (bf16) with_spmm_shape<__nv_bfloat16>(p.bh, nrhs, p.many, shape);
+    else with_spmm_shape<float>(p.bh, nrhs, p.many, shape);
+    const int rows = std::min(max_rows, (nbr + wave - 1) / wave);
+    const long long cap = nbr ? 2LL * rows * ((nblk + nbr - 1) / nbr) : 0;
     std::vector<int4> g;
     for (int r0 = 0, r1; r0 < nbr; r0 = r1) {
         for (r1 = r0 + 1; r1 < nbr && r1 - r0 < rows && rp[r1 + 1] - (long long)rp[r0] <= cap;) r1++;
@@ -873,12 +885,12 @@ static void launch_spmm(const Part& p, const float* x, float* y, int n, int k, b
     } else if (p.kind == PART_GBCSR && p.records) {
         const unsigned* rec = static_cast<const unsigned*>(p.v);
         if (p.nbr == 0) return;
-        with_spmm_shape<V>(p.bh, k, [&](auto sh) {
+        with_spmm_shape<V>(p.bh, k, p.many, [&](auto sh) {
             using Sh = decltype(sh);
             const unsigned g = grid_for((long long)p.nsgroups * Sh::GL, Sh::threads);
             auto launch = [&](auto kc) {
-                launch_chained(bcsr_spmm_stream_kernel<V, Sh::BH, Sh::BW, Sh::CW, decltype(kc)::value>, g, Sh::threads, 0, st, p.sgroups,
-                               p.nsgroups, p.i0, rec, x, y, p.m, k);
+                launch_chained(bcsr_spmm_stream_kernel<Sh, decltype(kc)::value>, g, Sh::threads, 0, st, p.sgroups, p.nsgroups, p.i0, rec,
+                               x, y, p.m, k);
             };
             if constexpr (Sh::CW <= 2) {
                 launch(std::integral_constant<int, 4 * Sh::CW>{});   // k is 4 or 8 here

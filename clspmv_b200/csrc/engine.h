@@ -44,6 +44,7 @@ struct Part {
     bool records = false;  // generic BCSR, k % 4 == 0: v holds block records (kernels/spmm.cuh)
     int4* sgroups = nullptr;        // their groups of block rows {first, end, first block, end block}
     int nsgroups = 0;
+    bool many = false;              // rows of many blocks (SpmmShape)
     int npad = 0, nwarps = 0;  // COO
     // x-panel layout (kernels/xpanel.cuh): i0 = run slot per entry, v = values
     unsigned short* lcol = nullptr;   // column inside the entry's panel

@@ -199,16 +199,22 @@ __device__ __forceinline__ void read_block(const unsigned* s, float (&a)[BS])
     }
 }
 
+// Whether a shape has a second kernel, for rows of many blocks (MANY below).
+constexpr bool spmm_has_many(int bw, int cw) { return (bw == 1 && cw != 2) || (bw == 2 && cw == 1); }
+
 // The lane split for CW float4 columns a pass.
-template <class V, int BH_, int BW_, int CW_> struct SpmmShape {
+template <class V_, int BH_, int BW_, int CW_, bool MANY = false> struct SpmmShape {
+    using V = V_;
     static constexpr int BH = BH_, BW = BW_, CW = CW_, BS = BH * BW;
     static constexpr int GL = 4 * CW, groups = 32 / GL;
     // rounds of X loads in flight: two, where 64 registers hold them; at one float4 column
-    // (k = 4) one for 3x3 and 4x4, which halves the ring and keeps more warps resident (197 ->
-    // 182 us); for 1x1, whose rounds are one load a lane, four (100,000 rows of 10 to 30 entries,
-    // one B200, before -> with four: k = 4 24.3 -> 17.1 us, k = 32 31.0 -> 29.3; 120,000 Zipf rows,
-    // k = 4 420 -> 118).  2x2, k = 4, 30,000 block rows: one 13.0, two 10.5
-    static constexpr int U = BW == 1 ? 4 : (BW > 4 || (BW > 2 && CW == 1) ? 1 : 2);
+    // (k = 4) one, which halves the ring and keeps more warps resident (3x3: 197 -> 182 us).  Small
+    // blocks of rows with many (MANY): four for 1x1, whose rounds are one load a lane, two for 2x2 at k = 4.
+    // 1x1, 200,000 rows, one B200, few / MANY: 3 entries a row, k = 32 24.6 / 33.7 us (rounds past a row's
+    // end are loads for nothing), 10 entries 39.4 / 37.7, k = 16 27.3 / 23.1; 100,000 rows of 10 to 30, k = 4
+    // 24.3 / 17.1; 120,000 Zipf rows, bound by the longest, k = 4 420 / 118.  At k = 8 MANY gains nothing
+    // (20,000 rows of 48: 8.9 / 11.1).  2x2, k = 4: 30,000 block rows of 10 to 30 13.0 / 10.5, 800,000 of 3 47.4 / 55.8
+    static constexpr int U = MANY ? (BW == 1 ? 4 : 2) : (BW > 4 || CW == 1 ? 1 : 2);
     static constexpr int chunk = 4 * U > 2 * CW ? 4 * U : 2 * CW;               // blocks; a step spans at most two
     static constexpr int ring_words = 4 * chunk * BlockRec<V, BS>::words;       // per group
     static constexpr int warp_bytes = groups * ring_words * 4;
@@ -224,13 +230,15 @@ template <class V, int BH_, int BW_, int CW_> struct SpmmShape {
     static constexpr int ctas = reg_ctas < smem_ctas ? reg_ctas : smem_ctas;
 };
 
-// K: the number of right-hand sides where it is known (0: `k_arg`).
-template <class V, int BH, int BW, int CW, int K>
-__global__ void __launch_bounds__(SpmmShape<V, BH, BW, CW>::threads, SpmmShape<V, BH, BW, CW>::ctas)
+// K: the number of right-hand sides where it is known (0: `k_arg`).  An instance of its own for k = 32
+// gains 4 to 12 % on 3x3 and 4x4 blocks over the one that takes any k above 16.
+template <class Sh, int K>
+__global__ void __launch_bounds__(Sh::threads, Sh::ctas)
     bcsr_spmm_stream_kernel(const int4* __restrict__ groups, int ngroups, const int* __restrict__ rp, const unsigned* __restrict__ rec,
                             const float* x, float* y, int m, int k_arg)
 {
-    using Sh = SpmmShape<V, BH, BW, CW>;
+    using V = typename Sh::V;
+    constexpr int BH = Sh::BH, BW = Sh::BW, CW = Sh::CW;
     using Rec = BlockRec<V, BH * BW>;
     constexpr int BS = BH * BW, GL = Sh::GL, U = Sh::U, CH = Sh::chunk, NW = Rec::words;
     constexpr int RM = 4 * CH - 1;   // ring index mask
