@@ -75,6 +75,17 @@ int Engine::alloc(void** p, size_t bytes)
     return CSP_OK;
 }
 
+// Gives back an array of alloc().
+void Engine::release(void* p)
+{
+    for (size_t i = 0; i < allocations.size(); i++)
+        if (allocations[i] == p) {
+            allocations.erase(allocations.begin() + i);
+            cudaFree(p);
+            return;
+        }
+}
+
 // Copies n host ints to a new device array of at least `cap` entries (zero tail).
 int Engine::upload_int(int** d, const int* h, size_t n, size_t cap)
 {
@@ -663,6 +674,7 @@ int Engine::add_bcsr(const b4csr_matrix_if& b, int method)
 int Engine::upload_block_records(Part& p, const bcsr_matrix_if& b)
 {
     constexpr size_t kHostWords = (size_t)128 << 10, kInlineBytes = (size_t)16 << 20, kSlice = (size_t)4 << 20;
+    const size_t before = device_bytes;
     const int bs = p.bw * p.bh;
     const size_t al = (size_t)b.bcsr_aligned_size, nblk = (size_t)b.bcsr_block_num, es = bf16 ? 2 : 4;
     const size_t words = dev::record_words(bs, bf16), total = (nblk + dev::kSpmmPadBlocks) * words;
@@ -691,7 +703,11 @@ int Engine::upload_block_records(Part& p, const bcsr_matrix_if& b)
     CSP_CUDA(cudaMemset(rec + nblk * words, 0, (size_t)dev::kSpmmPadBlocks * words * 4));
     char* tmp = reinterpret_cast<char*>(rec + total);
     cudaError_t e = inline_tmp ? cudaSuccess : cudaMalloc(reinterpret_cast<void**>(&tmp), tmp_bytes);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (block records)");
+    if (e != cudaSuccess) {
+        release(p.v);
+        device_bytes = before;
+        return cuda_error(e, "cudaMalloc (block records)");
+    }
     char* planes = tmp + slice * 4;
     // BF16 planes are converted together where they are small, else one after the other in one buffer
     const int group = inline_tmp ? bs : 1;
@@ -820,13 +836,21 @@ int Engine::add_generic_bcsr(const bcsr_matrix_if& b, int method)
     const int nblk = b.bcsr_block_num;
     if (nrhs % 4 == 0 && !(tensor_spmm && nrhs % 32 == 0 && bw * bh <= 16) && (long long)width * (nrhs / 4) <= UINT32_MAX) {
         // several right-hand sides in whole float4s, X rows indexed in 32 bits: block records
-        // (kernels/spmm.cuh)
-        if ((rc = upload_block_records(p, b)) || (rc = upload_spmm_groups(p, b.bcsr_row_ptr))) return rc;
-    } else if (!fits) {
+        // (kernels/spmm.cuh), where the device has room for them and their temporary
+        rc = upload_block_records(p, b);
+        if (rc && rc != CSP_ENOMEM) return rc;
+        if (rc) {
+            cudaGetLastError();
+            p.records = false;
+        } else if ((rc = upload_spmm_groups(p, b.bcsr_row_ptr))) {
+            return rc;
+        }
+    }
+    if (!p.records && !fits) {
         if ((rc = upload_int(&p.i1, b.bcsr_col_id, nblk, (size_t)pad_to(nblk, 4) + 4)) ||
             (rc = upload_val(&p.v, b.bcsr_data, nd, nd)))
             return rc;
-    } else {
+    } else if (fits) {
         // each item at a multiple of 4, its blocks in column order (stable) dealt to the
         // lanes of its 128-block chunks (kernels/block.cuh); tgt = row-order position - s,
         // 0xffff on empty slots

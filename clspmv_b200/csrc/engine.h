@@ -120,6 +120,7 @@ struct Engine {
     int launches_per_spmv() const;
 
     int alloc(void** p, size_t bytes);
+    void release(void* p);
     int upload_int(int** d, const int* h, size_t n, size_t cap);
     int upload_val(void** d, const float* h, size_t n, size_t cap);
 

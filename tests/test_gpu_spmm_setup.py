@@ -52,3 +52,35 @@ def test_time():
             hd.free()
         ms[k] = min(times)
     assert ms[4] <= 1.6 * ms[5], ms
+
+
+def test_device_nearly_full():
+    """1 M 3x3 blocks (40 MB of columns and planes) with 56 to 72 MB left on the device: no room for records
+    and their temporary, so the handle keeps the element planes, and the result is the same."""
+    k = 4
+    b, (h, w, r, c, v) = _bcsr(np.full(50_000, 20), 3, 14)
+    rng = np.random.default_rng(15)
+    X, Y0 = rng.uniform(-1, 1, (w, k)).astype(np.float32), rng.uniform(-1, 1, (h, k)).astype(np.float32)
+    small, _ = _bcsr(np.full(50, 20), 3, 16)
+    for n in (4, 5):   # loads the kernels of both layouts
+        hd = Handle(None, np.ones((9_003, n), np.float32), None, nrhs=n, bcsr=small)
+        hd.do_spmv(1)
+        hd.free()
+    torch.cuda.empty_cache()
+    fill, mib = [], 1 << 20
+    try:
+        fill.append(torch.empty(torch.cuda.mem_get_info()[0] - 66 * mib, dtype=torch.uint8, device="cuda"))
+        left = torch.cuda.mem_get_info()[0] // mib
+        assert 54 <= left <= 70, left
+        hd = Handle(None, X, Y0, nrhs=k, bcsr=b)
+        hd.do_spmv(1)
+        Y = hd.cpy_result_to_cpu().reshape(h, k)
+        hd.free()
+    finally:
+        fill.clear()
+        torch.cuda.empty_cache()
+    rp = csr_from_coo(h, r)
+    for j in range(k):
+        yhat, bound = _oracle.fp64_spmv(h, w, rp, c, v, np.ascontiguousarray(X[:, j]), np.ascontiguousarray(Y0[:, j]))
+        err, row = _oracle.max_rel_err(np.ascontiguousarray(Y[:, j]), yhat, bound)
+        assert err <= TOL, f"column {j}: error {err:.3e} at row {row}"
