@@ -382,9 +382,8 @@ std::vector<std::string> candidates(const Coo& a)
     if (h == w && nnz > 0) {
         // DIA only if the padded storage stays within the reference's 2x rule: a failed
         // conversion drops the DIA and BDIA candidates (see autotune_partition)
-        c.push_back("dia0");
+        // (every method runs the same kernel on the 32-aligned diagonals built here: one candidate a format)
         c.push_back("dia1");
-        c.push_back("bdia0");
         c.push_back("bdia1");
     }
     static const int bhs[4] = {1, 2, 4, 8};
