@@ -362,9 +362,9 @@ __device__ __forceinline__ void batch_dia(const BatchPart& P, int vb, int lane)
 }
 
 // BCSR block rows [vb * 16, vb * 16 + 16): kBatchBcsrLanes (2) lanes per block row,
-// each lane taking two of its row's blocks per round, whose column ids, values and x
-// gathers are all requested before any is used (the batch's block rows hold a few
-// blocks each: one or two rounds).
+// each lane taking one of its row's blocks per round, whose column id, values and x gathers
+// are all requested before any is used (the batch's block rows hold a few blocks each: one
+// to three rounds).
 template <class V, int B, bool GRAD>
 __device__ __forceinline__ void batch_bcsr(const BatchPart& P, int vb, int lane32)
 {
