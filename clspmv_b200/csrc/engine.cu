@@ -783,14 +783,20 @@ int Engine::upload_spmm_groups(Part& p, const int* rp)
     const int rows = std::min(max_rows, (nbr + wave - 1) / wave);
     const long long cap = nbr ? 2LL * rows * ((nblk + nbr - 1) / nbr) : 0;
     std::vector<int4> g;
+    bool cut = false;
     for (int r0 = 0, r1; r0 < nbr; r0 = r1) {
         for (r1 = r0 + 1; r1 < nbr && r1 - r0 < rows && rp[r1 + 1] - (long long)rp[r0] <= cap;) r1++;
         g.push_back(make_int4(r0, r1, rp[r0], rp[r1]));
+        cut = cut || (r1 - r0 < rows && r1 < nbr);
     }
     p.nsgroups = (int)g.size();
+    p.srows = rows;
+    // no group cut short: the kernel works the rows out, a dependent load less (10 M 3x3 blocks in BF16, k = 8:
+    // a pass of 206.2 us with the list, 204.5 without)
+    if (!cut) return CSP_OK;
     int rc = alloc(reinterpret_cast<void**>(&p.sgroups), g.size() * sizeof(int4));
     if (rc) return rc;
-    if (!g.empty()) CSP_CUDA(cudaMemcpy(p.sgroups, g.data(), g.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CSP_CUDA(cudaMemcpy(p.sgroups, g.data(), g.size() * sizeof(int4), cudaMemcpyHostToDevice));
     return CSP_OK;
 }
 
@@ -936,8 +942,8 @@ static void launch_spmm(const Part& p, const float* x, float* y, int n, int k, b
             using Sh = decltype(sh);
             const unsigned g = grid_for((long long)p.nsgroups * Sh::GL, Sh::threads);
             auto launch = [&](auto kc) {
-                launch_chained(bcsr_spmm_stream_kernel<Sh, decltype(kc)::value>, g, Sh::threads, 0, st, p.sgroups, p.nsgroups, p.i0, rec,
-                               x, y, p.m, k);
+                launch_chained(bcsr_spmm_stream_kernel<Sh, decltype(kc)::value>, g, Sh::threads, 0, st, p.sgroups, p.nsgroups, p.srows, p.i0,
+                               rec, x, y, p.nbr, p.m, k);
             };
             if constexpr (Sh::CW <= 2) {
                 launch(std::integral_constant<int, 4 * Sh::CW>{});   // k is 4 or 8 here

@@ -42,7 +42,8 @@ struct Part {
     int group = 0;    // CSR sub-warp lanes per row
     int nblocks = 0;  // CSR adaptive row blocks
     bool records = false;  // generic BCSR, k % 4 == 0: v holds block records (kernels/spmm.cuh)
-    int4* sgroups = nullptr;        // their groups of block rows {first, end, first block, end block}
+    int srows = 0;                  // block rows of one lane group, all alike
+    int4* sgroups = nullptr;        // or, where they differ, their {first, end, first block, end block}
     int nsgroups = 0;
     bool many = false;              // rows of many blocks (SpmmShape)
     int npad = 0, nwarps = 0;  // COO

@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(kSpmmThreads) bcsr_spmm_kernel(const int* __re
 // Generic BCSR with k a multiple of 4, on a layout of its own: block j is BlockRec<V, BS>
 // words -- its BS values in row-major order (two per word in BF16), then the index of
 // its first X row in float4s -- so a run of blocks is one contiguous stream.  A warp is
-// cut into groups of GL = 4 CW lanes; a group takes consecutive block rows (the host's
-// `groups`: at most max_rows, and at most one where a row is long) one after the other and copies their blocks through a ring of four chunks in shared memory
+// cut into groups of GL = 4 CW lanes; a group takes `rows` consecutive block rows, or those of the
+// host's list `groups` where some rows are long, one after the other and copies their blocks through a ring of four chunks in shared memory
 // with 16-byte cp.async, two chunks ahead.  Per step a group takes 4 U blocks of its
 // current row: lane (cw, sub) owns right-hand sides 4 cw .. 4 cw + 3 of blocks sub,
 // sub + 4, ..., whose X loads are all in flight together.  At the end of a row the four
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kSpmmThreads) bcsr_spmm_kernel(const int* __re
 // path and the L1 tag rate (BW lines a block at a line a clock), not HBM; next to it, issue
 // slots: BH * BW * 4 FMAs per lane and block, and as few other instructions as possible --
 // no predicated loads (lanes past the row's end read X row 0 and skip the products).
-// Measured (500,000 block rows, 10 M 3x3 blocks, one B200): k = 32 FP32 615 -> 355 us, k = 16
+// Measured (500,000 block rows, 10 M 3x3 blocks, one B200): k = 32 FP32 615 -> 344 us, k = 16
 // 530 -> 271, k = 8 BF16 250 -> 187, k = 4 FP32 245 -> 182 (before: blocks staged row by row
 // from the element planes, one barrier pair per 32 blocks, ~880 instructions a block row at
 // k = 32; now ~580).  The X gathers alone take 192 us at k = 32.  Also measured at k = 32:
@@ -234,8 +234,8 @@ template <class V_, int BH_, int BW_, int CW_, bool MANY = false> struct SpmmSha
 // gains 4 to 12 % on 3x3 and 4x4 blocks over the one that takes any k above 16.
 template <class Sh, int K>
 __global__ void __launch_bounds__(Sh::threads, Sh::ctas)
-    bcsr_spmm_stream_kernel(const int4* __restrict__ groups, int ngroups, const int* __restrict__ rp, const unsigned* __restrict__ rec,
-                            const float* x, float* y, int m, int k_arg)
+    bcsr_spmm_stream_kernel(const int4* __restrict__ groups, int ngroups, int rows, const int* __restrict__ rp,
+                            const unsigned* __restrict__ rec, const float* x, float* y, int nbr, int m, int k_arg)
 {
     using V = typename Sh::V;
     constexpr int BH = Sh::BH, BW = Sh::BW, CW = Sh::CW;
@@ -250,9 +250,15 @@ __global__ void __launch_bounds__(Sh::threads, Sh::ctas)
     unsigned* ring = s_ring[threadIdx.x / GL];
     const unsigned ring_addr = (unsigned)__cvta_generic_to_shared(ring);
     const int gid = (int)(((long long)blockIdx.x * Sh::threads + threadIdx.x) / GL);
-    // block rows [x, y) with blocks [z, w)
-    const int4 gr = gid < ngroups ? __ldg(groups + gid) : make_int4(0, 0, 0, 0);
-    const int r0 = gr.x, r1 = gr.y, sb = gr.z, eb = gr.w;
+    // block rows [r0, r1) with blocks [sb, eb)
+    int r0, r1, sb, eb;
+    if (groups) {
+        const int4 gr = gid < ngroups ? __ldg(groups + gid) : make_int4(0, 0, 0, 0);
+        r0 = gr.x, r1 = gr.y, sb = gr.z, eb = gr.w;
+    } else {
+        r0 = (int)min((long long)gid * rows, (long long)nbr), r1 = min(r0 + rows, nbr);
+        sb = __ldg(rp + r0), eb = __ldg(rp + r1);
+    }
     const int cw = lane % CW, sub = lane / CW;
     const int rend = __ldg(rp + min(r0 + 1 + lane, r1));     // rows <= GL: the ends of the group's rows
     const int base = sb & ~1;                                // chunks start on 16 bytes
