@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kSpmmThreads) bcsr_spmm_kernel(const int* __re
 // path and the L1 tag rate (BW lines a block at a line a clock), not HBM; next to it, issue
 // slots: BH * BW * 4 FMAs per lane and block, and as few other instructions as possible --
 // no predicated loads (lanes past the row's end read X row 0 and skip the products).
-// Measured (500,000 block rows, 10 M 3x3 blocks, one B200): k = 32 FP32 615 -> 344 us, k = 16
+// Measured (500,000 block rows, 10 M 3x3 blocks, one B200): k = 32 FP32 615 -> 342 us, k = 16
 // 530 -> 271, k = 8 BF16 250 -> 187, k = 4 FP32 245 -> 182 (before: blocks staged row by row
 // from the element planes, one barrier pair per 32 blocks, ~880 instructions a block row at
 // k = 32; now ~580).  The X gathers alone take 192 us at k = 32.  Also measured at k = 32:
