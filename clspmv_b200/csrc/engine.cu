@@ -1324,8 +1324,27 @@ int Engine::init_common(int w, int h, int nz, int flags, int k)
     return CSP_OK;
 }
 
-// x, y and, where csp_iterate's steps alternate (`steps`), its second vector behind x (in one
-// allocation: a second one adds 0.1-0.3 ms to the set-up).  Called once the parts are known.
+// Whether a cocktail is one part that covers every row with a kernel that takes the accumulated
+// vector and the result apart (has_step); told from the caller's structs, before any part is built.
+// It is also true for wide BF16 bands that will run the staged kernel.
+static bool one_step_part(const cocktail_iif* c)
+{
+    const int h = c->mat_height;
+    const int used = c->ifusebdia + c->ifusedia + c->ifusesbell + c->ifusebell + c->ifusebcsr + c->ifusesell + c->ifuseell +
+                     c->ifusecsr + c->ifusecoo;
+    if (used != 1 || c->mat_width != h || h <= 0) return false;
+    if (c->ifusecsr) return c->csr_meth_num == 2 && c->csr.matinfo.height == h;
+    if (c->ifuseell) return c->ell_meth_num == 1 && c->ell.ell_height_aligned % 4 == 0 && c->ell.matinfo.height == h;
+    if (c->ifusedia) return c->dia.dia_length_aligned % 4 == 0 && std::min(c->dia.matinfo.height, c->dia.dia_length_aligned) >= h;
+    if (c->ifusebdia)
+        return c->bdia.bdia_length_aligned % 4 == 0 && std::min(c->bdia.matinfo.height, c->bdia.bdia_length_aligned) >= h;
+    return false;
+}
+
+// x, y and, where csp_iterate's steps may alternate (`steps`), its second vector behind x (in one
+// allocation: a second one adds 0.1-0.3 ms to the set-up).  They come before the parts: behind them
+// small random gathers are slower (50,000 rows of 40 entries as CSR, one B200: 10.4 us before the
+// parts, 12.1 behind them).
 int Engine::init_vectors(const float* vec, const float* res, int flags, bool steps)
 {
     const size_t x_floats = (size_t)x_len * nrhs * (steps ? 2 : 1);
@@ -1360,6 +1379,7 @@ int Engine::init(const cocktail_iif* mat, const float* vec, const float* res, in
             return set_error(CSP_EUNSUP, "several right-hand sides need blocks of <= 36 elements");
         if (flags & CSP_FLAG_ADJOINT) return set_error(CSP_EUNSUP, "adjoint with several right-hand sides");
     }
+    if ((rc = init_vectors(vec, res, flags, nrhs == 1 && one_step_part(mat)))) return rc;
     // parts, in the reference's launch order
     if (mat->ifusebdia && (rc = add_bdia(mat->bdia))) return rc;
     if (mat->ifusedia && (rc = add_dia(mat->dia))) return rc;
@@ -1376,8 +1396,7 @@ int Engine::init(const cocktail_iif* mat, const float* vec, const float* res, in
     if (mat->ifusecsr && (rc = add_csr(mat->csr, mat->csr_meth_num))) return rc;
     if (mat->ifusecoo && (rc = add_coo(mat->coo, mat->coo_meth_num))) return rc;
     if ((flags & CSP_FLAG_ADJOINT) && (rc = build_adjoint(mat))) return rc;
-    const bool steps = width == height && nrhs == 1 && parts.size() == 1 && has_step(parts[0]) && parts[0].m == height && height > 0;
-    if ((rc = init_vectors(vec, res, flags, steps))) return rc;
+    if (!(parts.size() == 1 && has_step(parts[0]) && parts[0].m == height)) d_z = nullptr;
     CSP_CUDA(cudaDeviceSynchronize());
     return CSP_OK;
 }
@@ -1389,9 +1408,8 @@ int Engine::init_bcsr(const bcsr_matrix_if* b, const float* vec, const float* re
     if (k > 1 && b->bcsr_bwidth * b->bcsr_bheight > 36) return set_error(CSP_EUNSUP, "several right-hand sides need blocks of <= 36 elements");
     int rc = init_common(b->matinfo.width, b->matinfo.height, b->matinfo.nnz, flags, k);
     if (rc) return rc;
-    if ((rc = add_generic_bcsr(*b, 0))) return rc;
+    if ((rc = init_vectors(vec, res, flags, false)) || (rc = add_generic_bcsr(*b, 0))) return rc;
     if ((flags & CSP_FLAG_ADJOINT) && (rc = build_adjoint_gbcsr(*b))) return rc;
-    if ((rc = init_vectors(vec, res, flags, false))) return rc;
     CSP_CUDA(cudaDeviceSynchronize());
     return CSP_OK;
 }
